@@ -140,6 +140,7 @@ static void free_plan(cunusht_plan_s *P) {
             if (P->d_tc_stv[g][s]) cudaFree(P->d_tc_stv[g][s]);
             if (P->d_tc_ste[g][s]) cudaFree(P->d_tc_ste[g][s]);
         }
+    if (P->d_t6_slab) cudaFree(P->d_t6_slab);
     for (auto &e : P->evt_pool) {
         cudaEventDestroy(e.a);
         cudaEventDestroy(e.b);
@@ -247,6 +248,7 @@ static int build_plan(cunusht_plan_s *P, int lmax, double eps, int precision, in
                 set_error("pointing geometry is not north/south symmetric (ring %g vs %g)", tn, ts);
                 return CUNUSHT_ERR_UNSUPPORTED;
             }
+            P->h_gl_theta.push_back(tn);
             x.push_back(std::cos(tn));
             sh.push_back(std::sin(0.5 * tn));
             ch.push_back(std::cos(0.5 * tn));
@@ -304,6 +306,7 @@ static int build_plan(cunusht_plan_s *P, int lmax, double eps, int precision, in
         std::vector<int> rn, rs;
         for (int k = 0; k <= P->Nt / 4; ++k) {
             const double t = TWOPI * k / P->Nt;
+            P->h_cc_theta.push_back(t);
             x.push_back(std::cos(t));
             sh.push_back(std::sin(0.5 * t));
             ch.push_back(std::cos(0.5 * t));
@@ -344,6 +347,7 @@ static int build_plan(cunusht_plan_s *P, int lmax, double eps, int precision, in
     RC_TRY(dalloc(P, &P->d_status, 1));
     CU_TRY(cudaMemset(P->d_status, 0, sizeof(int)));
     if (P->prec == CUNUSHT_PREC_MIXED) RC_TRY(tc_plan_init(P));
+    else RC_TRY(tc64_plan_init(P));
     {
         std::vector<double> lf(lmax + 1);
         for (int l = 0; l <= lmax; ++l) lf[l] = std::sqrt((double)l * (l + 1.0));

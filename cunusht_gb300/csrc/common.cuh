@@ -151,6 +151,11 @@ constexpr int MR_NMAX = 8192;
 constexpr int MR_MAXST = 16;
 constexpr int MR_KMAX = 128;
 
+// log2 sin(theta/2) and log2 cos(theta/2) of a ring as FP64 pairs (high part -inf for a zero)
+struct RingLog {
+    double sh, sl, ch, cl;
+};
+
 struct cunusht_plan_s {
     int lmax = 0;
     int max_spin = 0;
@@ -201,7 +206,7 @@ struct cunusht_plan_s {
     double *d_lg0[3] = {nullptr, nullptr, nullptr};  // per m: log2 start normalisation
     double *d_lfac = nullptr;                        // sqrt(l(l+1)), l = 0..L
     float2 *d_coef_df[3] = {nullptr, nullptr, nullptr};  // the same tables as (hi, lo) FP32 pairs
-    bool use_tc = true;       // mixed precision: Legendre synthesis (every spin) on the tensor cores
+    bool use_tc = true;       // Legendre stages (every spin) on the tensor cores
     int *d_status = nullptr;  // device status word: bit 0 = a bounded wait of a tensor-core kernel ran out
     // tensor-core synthesis: per spin 1, 2 the first window record of each m (m = 0..lmax+1),
     // and the record buffer (alm digit planes and scales per (m, l-window), written per call)
@@ -215,6 +220,21 @@ struct cunusht_plan_s {
     // (NULL: the kernel evaluates the start itself)
     float4 *d_tc_stv[2][3] = {};
     short2 *d_tc_ste[2][3] = {};
+
+    // FP64 plans on the tensor cores (legendre_tc64.cu): rescaled recursion (a_l, g_l) and the
+    // scale c_l per spin, start states (value, previous value), (exponent / 512, first chunk of
+    // 16 l) per [grid: 0 GL, 1 CC][spin], window offsets and records as above; one allocation
+    void *d_t6_slab = nullptr;
+    unsigned char *d_t6_rec = nullptr;
+    int *d_t6_woff[3] = {};
+    double2 *d_t6_ag[3] = {};
+    double *d_t6_cl[3] = {};
+    short *d_t6_eb[3] = {};     // digit exponent of mu per (m, chunk of 16 l)
+    double2 *d_t6_lg0[3] = {};  // per m: log2 start normalisation (hi, lo)
+    RingLog *d_t6_lsc[2] = {};  // per [grid][pair]: log2 sin(theta/2), log2 cos(theta/2), (hi, lo) each
+    std::vector<double> h_gl_theta, h_cc_theta;  // theta of the ring pairs
+    double2 *d_t6_stv[2][3] = {};
+    short2 *d_t6_ste[2][3] = {};
 
     // FFT twiddles e^{-2 pi i t / TW}
     int TW = 0;

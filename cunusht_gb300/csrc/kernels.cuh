@@ -60,6 +60,30 @@ int leg_synth_spin_tc(const cunusht_plan_s *P, int nb, int npairs, const double 
                       const float4 *stv, const short2 *ste, int spin, const double2 *G,
                       const double2 *C, long long astride, const double *lf, double2 *H, long long hstride,
                       cudaStream_t st);
+// the pole pair (theta = 0, pi) of a synthesis in closed form
+int leg_synth_pole_pair(const cunusht_plan_s *P, int nreq, int spin, const double2 *G, const double2 *C,
+                        long long astride, const double *lf, int rn, int rs, double2 *H, long long hstride, int ld,
+                        cudaStream_t st);
+// legendre_tc64.cu: tensor-core synthesis of the FP64 plans (one request)
+int tc64_plan_init(cunusht_plan_s *P);
+int leg_synth_tc64(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
+                   const int *rn, const int *rs, int ld, int pole, int pole_rn, int pole_rs, bool cc, int spin,
+                   const double2 *G, const double2 *C, const double *lf, double2 *H, cudaStream_t st);
+// legendre_tc64_adj.cu: tensor-core adjoint of the FP64 plans (one request, alm zeroed by the caller)
+int leg_adjoint_tc64(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
+                     const int *rn, const int *rs, int ld, int pole, int pole_rn, int pole_rs, bool cc, int spin,
+                     int ncomp, const double2 *H, const double *lf, double2 *G, double2 *C, cudaStream_t st);
+int leg_adj_f64_pairs(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
+                      const int *rn, const int *rs, int ld, int spin, int ncomp, const double2 *H, const double *lf,
+                      double2 *G, double2 *C, cudaStream_t st);
+// the pole pair of an adjoint, added to the alm
+int leg_adj_pole_pair(const cunusht_plan_s *P, int nreq, int spin, int ncomp, const double2 *H, long long hstride,
+                      int ld, const double *lf, int rn, int rs, double2 *G, double2 *C, long long astride,
+                      cudaStream_t st);
+// legendre.cu: FP64 CUDA-core synthesis of npairs ring pairs given by their tables
+int leg_synth_f64_pairs(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
+                        const int *rn, const int *rs, int ld, int spin, const double2 *G, const double2 *C,
+                        const double *lf, double2 *H, cudaStream_t st);
 int tc_selftest(int nn, int reps, int mode, double *maxerr, int *timeout);
 int tc_plan_init(cunusht_plan_s *P);  // window tables and record buffer of a mixed-precision plan
 int tc_start_states(cunusht_plan_s *P, int grid, int spin, bool enable);  // build / release one start-state table

@@ -27,40 +27,9 @@
 #include "common.cuh"
 #include "df.cuh"
 #include "kernels.cuh"
+#include "rec64.cuh"
 
 namespace cunusht {
-
-__device__ __forceinline__ void rec_start(double lg0, int m, int s, double sh, double ch,
-                                          double &cur, double &prev, int &e) {
-    prev = 0.0;
-    double lg = lg0;
-    bool zero = false;
-    if (m + s > 0) {
-        if (sh <= 0.0) zero = true;
-        else lg += (double)(m + s) * log2(sh);
-    }
-    if (m != s) {
-        if (ch <= 0.0) zero = true;
-        else lg += (double)abs(m - s) * log2(ch);
-    }
-    if (zero) {
-        cur = 0.0;
-        e = 0;
-        return;
-    }
-    int k = 0;
-    if (lg < -400.0) k = (int)ceil((-400.0 - lg) / 512.0);
-    e = -512 * k;
-    cur = exp2(lg + 512.0 * (double)k);
-    if (m & 1) cur = -cur;
-}
-
-#define REC_RESCALE(cur, prev, e)                                                        \
-    if ((e) < 0 && fabs(cur) > 0x1p200) {                                               \
-        (cur) *= 0x1p-512;                                                               \
-        (prev) *= 0x1p-512;                                                              \
-        (e) += 512;                                                                      \
-    }
 
 // ---------------------------------------------------------------- tables
 __global__ void k_build_coef(int L, int s, double *__restrict__ coef, long long nalm) {
@@ -1166,16 +1135,27 @@ int leg_synth_batch_fl(const cunusht_plan_s *P, int nreq, int spin, const double
     for (int r = 0; r < nreq; ++r) {
         const double2 *Gr = G + r * astride, *Cr = C ? C + r * astride : nullptr;
         double2 *Hr = H + r * hstride;
-        if (spin == 0) {
-            k_leg_synth_s0<<<grid, LEG_TPB, 0, st>>>(L, Gr, lf, P->d_coef[0], P->nalm_tab, P->d_lg0[0], R.npairs, R.x,
-                                                     R.sh, R.ch, R.rn, R.rs, Hr, R.ld);
-        } else {
-            k_leg_synth_spin<<<grid, LEG_TPB, 0, st>>>(L, spin, Gr, Cr, lf, P->d_coef[spin], P->nalm_tab,
-                                                       P->d_lg0[spin], R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, Hr,
-                                                       R.ld);
-        }
-        CU_LAUNCH_CHECK();
+        if (P->use_tc && P->d_t6_ag[spin])
+            RC_TRY(leg_synth_tc64(P, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.ld, R.pole, R.pole_rn, R.pole_rs, cc,
+                                  spin, Gr, Cr, lf, Hr, st));
+        else
+            RC_TRY(leg_synth_f64_pairs(P, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.ld, spin, Gr, Cr, lf, Hr, st));
     }
+    return CUNUSHT_OK;
+}
+
+int leg_synth_f64_pairs(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
+                        const int *rn, const int *rs, int ld, int spin, const double2 *G, const double2 *C,
+                        const double *lf, double2 *H, cudaStream_t st) {
+    const int L = P->lmax;
+    const dim3 grid((npairs + LEG_TPB - 1) / LEG_TPB, P->mmax + 1);
+    if (spin == 0)
+        k_leg_synth_s0<<<grid, LEG_TPB, 0, st>>>(L, G, lf, P->d_coef[0], P->nalm_tab, P->d_lg0[0], npairs, x, sh, ch,
+                                                 rn, rs, H, ld);
+    else
+        k_leg_synth_spin<<<grid, LEG_TPB, 0, st>>>(L, spin, G, C, lf, P->d_coef[spin], P->nalm_tab, P->d_lg0[spin],
+                                                   npairs, x, sh, ch, rn, rs, H, ld);
+    CU_LAUNCH_CHECK();
     return CUNUSHT_OK;
 }
 
@@ -1317,16 +1297,28 @@ int leg_adjoint_batch(const cunusht_plan_s *P, int nreq, int spin, int ncomp, co
     for (int r = 0; r < nreq; ++r) {
         const double2 *Hr = H + r * hstride;
         double2 *Gr = G + r * astride, *Cr = (spin > 0 && ncomp > 1) ? C + r * astride : nullptr;
-        if (spin == 0) {
-            k_leg_adj_s0<<<grid, LEG_TPB, 0, st>>>(L, Hr, R.ld, lf, P->d_coef[0], P->nalm_tab, P->d_lg0[0], R.npairs,
-                                                   R.x, R.sh, R.ch, R.rn, R.rs, (double *)Gr);
-        } else {
-            k_leg_adj_spin<<<grid, LEG_TPB, 0, st>>>(L, spin, ncomp, Hr, R.ld, lf, P->d_coef[spin], P->nalm_tab,
-                                                     P->d_lg0[spin], R.npairs, R.x, R.sh, R.ch, R.rn, R.rs,
-                                                     (double *)Gr, (double *)Cr);
-        }
-        CU_LAUNCH_CHECK();
+        if (P->use_tc && P->d_t6_ag[spin])
+            RC_TRY(leg_adjoint_tc64(P, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.ld, R.pole, R.pole_rn, R.pole_rs, cc,
+                                    spin, ncomp, Hr, lf, Gr, Cr, st));
+        else
+            RC_TRY(leg_adj_f64_pairs(P, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.ld, spin, ncomp, Hr, lf, Gr, Cr,
+                                     st));
     }
+    return CUNUSHT_OK;
+}
+
+int leg_adj_f64_pairs(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
+                      const int *rn, const int *rs, int ld, int spin, int ncomp, const double2 *H, const double *lf,
+                      double2 *G, double2 *C, cudaStream_t st) {
+    const int L = P->lmax;
+    const dim3 grid((npairs + LEG_TPB - 1) / LEG_TPB, P->mmax + 1);
+    if (spin == 0)
+        k_leg_adj_s0<<<grid, LEG_TPB, 0, st>>>(L, H, ld, lf, P->d_coef[0], P->nalm_tab, P->d_lg0[0], npairs, x, sh, ch,
+                                               rn, rs, (double *)G);
+    else
+        k_leg_adj_spin<<<grid, LEG_TPB, 0, st>>>(L, spin, ncomp, H, ld, lf, P->d_coef[spin], P->nalm_tab,
+                                                 P->d_lg0[spin], npairs, x, sh, ch, rn, rs, (double *)G, (double *)C);
+    CU_LAUNCH_CHECK();
     return CUNUSHT_OK;
 }
 

@@ -1026,6 +1026,18 @@ __global__ void __launch_bounds__(POLE_TPB)
     }
 }
 
+int leg_synth_pole_pair(const cunusht_plan_s *P, int nreq, int spin, const double2 *G, const double2 *C,
+                        long long astride, const double *lf, int rn, int rs, double2 *H, long long hstride, int ld,
+                        cudaStream_t st) {
+    if (spin == 0)
+        k_pole_pair_s0<<<nreq, POLE_TPB, 0, st>>>(P->lmax, P->mmax, G, astride, lf, rn, rs, H, hstride, ld);
+    else
+        k_pole_pair_spin<<<nreq, POLE_TPB, 0, st>>>(P->lmax, spin, P->mmax, G, C, astride, lf, rn, rs, H, hstride,
+                                                    ld);
+    CU_LAUNCH_CHECK();
+    return CUNUSHT_OK;
+}
+
 // Ring pairs in full blocks (256 pairs, 128 for NB = 8; spin 0: 512 and 256) on the tensor cores; a
 // tail of fewer than TCL_MIN_TAIL pairs after at least one full block goes to
 // the double-float CUDA-core kernel instead of a nearly empty block per order m.
@@ -1037,13 +1049,7 @@ int leg_synth_spin_tc(const cunusht_plan_s *P, int nb, int npairs, const double 
     if (pole == 0 && npairs > 1) {
         // the pole pair in closed form; the tensor cores take the other pairs
         // (a Clenshaw-Curtis grid of 2^k + 1 rings then fills whole blocks)
-        if (spin == 0)
-            k_pole_pair_s0<<<nb, POLE_TPB, 0, st>>>(P->lmax, P->mmax, G, astride, lf, pole_rn, pole_rs, H, hstride,
-                                                    ld);
-        else
-            k_pole_pair_spin<<<nb, POLE_TPB, 0, st>>>(P->lmax, spin, P->mmax, G, C, astride, lf, pole_rn, pole_rs,
-                                                      H, hstride, ld);
-        CU_LAUNCH_CHECK();
+        RC_TRY(leg_synth_pole_pair(P, nb, spin, G, C, astride, lf, pole_rn, pole_rs, H, hstride, ld, st));
         ++x, ++sh, ++ch, ++rn, ++rs;
         if (stv) ++stv, ++ste;
         --npairs;

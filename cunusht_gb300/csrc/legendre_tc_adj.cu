@@ -502,6 +502,17 @@ __global__ void k_pole_pair_adj_s0(int L, const double2 *__restrict__ H, long lo
     }
 }
 
+int leg_adj_pole_pair(const cunusht_plan_s *P, int nreq, int spin, int ncomp, const double2 *H, long long hstride,
+                      int ld, const double *lf, int rn, int rs, double2 *G, double2 *C, long long astride,
+                      cudaStream_t st) {
+    if (spin)
+        return leg_adj_pole_pair_spin(P, nreq, spin, ncomp, H, hstride, ld, lf, rn, rs, G, C, astride, st);
+    k_pole_pair_adj_s0<<<dim3((P->lmax + 256) / 256, nreq), 256, 0, st>>>(P->lmax, H, hstride, lf, rn, rs, (double *)G,
+                                                                          astride);
+    CU_LAUNCH_CHECK();
+    return CUNUSHT_OK;
+}
+
 template <int NB, bool S0>
 static int launch_adj_tc_nb(const cunusht_plan_s *P, const TcAdjArgs &A, int r0, cudaStream_t st) {
     CU_TRY(cudaFuncSetAttribute(k_leg_adj_tc<NB, S0>, cudaFuncAttributeMaxDynamicSharedMemorySize, TCA_BYTES));
@@ -572,16 +583,7 @@ int leg_adjoint_tc(const cunusht_plan_s *P, int nreq, int spin, int ncomp, const
         L, spin, ncomp, A.acc, P->nalm_tab, A.hm, A.npairs_all, lf, (double *)G,
         (spin > 0 && ncomp > 1) ? (double *)C : nullptr, astride);
     CU_LAUNCH_CHECK();
-    if (has_pole) {
-        if (spin == 0) {
-            k_pole_pair_adj_s0<<<dim3((L + 256) / 256, nreq), 256, 0, st>>>(L, H, hstride, lf, pole_rn, pole_rs,
-                                                                            (double *)G, astride);
-            CU_LAUNCH_CHECK();
-        } else {
-            RC_TRY(leg_adj_pole_pair_spin(P, nreq, spin, ncomp, H, hstride, ld, lf, pole_rn, pole_rs, G, C, astride,
-                                          st));
-        }
-    }
+    if (has_pole) RC_TRY(leg_adj_pole_pair(P, nreq, spin, ncomp, H, hstride, ld, lf, pole_rn, pole_rs, G, C, astride, st));
     if (A.ntc < npairs)
         RC_TRY(leg_adj_df_pairs(P, nreq, spin, ncomp, H, hstride, ld, npairs - A.ntc, x + A.ntc, sh + A.ntc,
                                 ch + A.ntc, rn + A.ntc, rs + A.ntc, lf, G, C, astride, st));
