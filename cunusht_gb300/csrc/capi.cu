@@ -125,7 +125,7 @@ static void free_plan(cunusht_plan_s *P) {
     void *ptrs[] = {P->d_ring_sc, P->d_ring_theta, P->d_ring_phi0, P->d_ring_nph, P->d_ring_ofs, P->d_gl_x, P->d_gl_sh,
                     P->d_gl_ch, P->d_gl_rn, P->d_gl_rs, P->d_cc_x, P->d_cc_sh, P->d_cc_ch, P->d_cc_rn,
                     P->d_cc_rs, P->d_Dth, P->d_Dph, P->d_coef[0], P->d_coef[1], P->d_coef[2], P->d_lg0[0],
-                    P->d_lg0[1], P->d_lg0[2], P->d_lfac, P->d_coef_df[0], P->d_coef_df[1], P->d_coef_df[2], P->d_tw64, P->d_tw32, P->d_twdf, P->d_chirp_df, P->d_bker_df, P->d_chirp, P->d_bker,
+                    P->d_lg0[1], P->d_lg0[2], P->d_lfac, P->d_tc_co[0], P->d_tc_co[1], P->d_tc_co[2], P->d_tw64, P->d_tw32, P->d_twdf, P->d_chirp_df, P->d_bker_df, P->d_chirp, P->d_bker,
                     P->d_H, P->d_F, P->d_U, P->d_Hgl, P->d_ring, P->d_glmap, P->d_alm, P->d_vjp, P->d_lfac_g, P->d_ring_cls, P->d_cls_N, P->d_cls_Mb, P->d_cls_SP,
                     P->d_cls_coff, P->d_cls_boff, P->d_Hb, P->d_Fb, P->d_Ub,  // d_Hglb, d_glmapb alias d_Hb, d_Fb
                     P->d_ptgb, P->d_gamb, P->d_status, P->d_tc_woff[0], P->d_tc_woff[1], P->d_tc_woff[2],
@@ -341,8 +341,7 @@ static int build_plan(cunusht_plan_s *P, int lmax, double eps, int precision, in
     }
     RC_TRY(build_coef_tables(P, 0));
     if (P->prec == CUNUSHT_PREC_MIXED) {
-        for (int s = 0; s <= 2; ++s) RC_TRY(dalloc(P, &P->d_coef_df[s], 3 * (size_t)P->nalm_tab));
-        RC_TRY(build_coef_tables_df(P, 0));
+        RC_TRY(build_coef_tables_df(P));
     }
     RC_TRY(dalloc(P, &P->d_status, 1));
     CU_TRY(cudaMemset(P->d_status, 0, sizeof(int)));

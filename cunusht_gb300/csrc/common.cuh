@@ -205,12 +205,11 @@ struct cunusht_plan_s {
     double *d_coef[3] = {nullptr, nullptr, nullptr};
     double *d_lg0[3] = {nullptr, nullptr, nullptr};  // per m: log2 start normalisation
     double *d_lfac = nullptr;                        // sqrt(l(l+1)), l = 0..L
-    float2 *d_coef_df[3] = {nullptr, nullptr, nullptr};  // the same tables as (hi, lo) FP32 pairs
+    float *d_tc_co[3] = {};   // mixed plans: the same as double-floats, in windows of 128 l (rec64.cuh co_load)
+    int *d_tc_woff[3] = {};   // first window of each m (m = 0..lmax+1)
     bool use_tc = true;       // Legendre stages (every spin) on the tensor cores
     int *d_status = nullptr;  // device status word: bit 0 = a bounded wait of a tensor-core kernel ran out
-    // tensor-core synthesis: per spin 1, 2 the first window record of each m (m = 0..lmax+1),
-    // and the record buffer (alm digit planes and scales per (m, l-window), written per call)
-    int *d_tc_woff[3] = {nullptr, nullptr, nullptr};
+    // tensor-core synthesis: record buffer (alm digit planes and scales per (m, l-window), written per call)
     unsigned char *d_tc_rec = nullptr;
     size_t tc_rec_bytes = 0;
     size_t tc_nrec = 0;  // window records per call (the larger of spin 1 and 2)

@@ -172,9 +172,6 @@ __device__ __forceinline__ dfl df_mul_u(dfl a, dfl x) {
     return dfl{p, e};
 }
 
-// a * x + g as an unnormalised pair: 12 operations instead of 18 (df_mul, df_add)
-__device__ __forceinline__ dfl df_fma_u(dfl a, dfl x, dfl g) { return df_add_u(df_mul_u(a, x), g); }
-
 // t * x - b * y, renormalised (t may be unnormalised)
 __device__ __forceinline__ dfl df_mul_sub(dfl t, dfl x, dfl b, dfl y) {
     const dfl p1 = df_mul_u(t, x), p2 = df_mul_u(b, y);
@@ -182,6 +179,77 @@ __device__ __forceinline__ dfl df_mul_sub(dfl t, dfl x, dfl b, dfl y) {
     const float bb = s - p1.h;
     const float err = (p1.h - (s - bb)) + (-p2.h - bb);
     return df_fast(s, err + (p1.l - p2.l));
+}
+
+// t = a x + g (no g: a x), unnormalised, in the operations and order of df2_factor
+template <bool G> __device__ __forceinline__ dfl df_factor(dfl a, dfl x, dfl g) {
+    const float np = __fmul_rn(a.h, -x.h);
+    float e = __fmaf_rn(a.h, x.h, np);
+    e = __fmaf_rn(a.h, x.l, e);
+    e = __fmaf_rn(a.l, x.h, e);
+    if (!G) return dfl{-np, e};
+    const float s = __fsub_rn(g.h, np);
+    const float bb = __fsub_rn(s, g.h);
+    const float err = __fsub_rn(__fsub_rn(g.h, __fsub_rn(s, bb)), __fadd_rn(np, bb));
+    return dfl{s, __fadd_rn(__fadd_rn(e, g.l), err)};
+}
+
+// Two FP32 values in one 64-bit register pair: the packed f32x2 instructions
+// do two lanes' work in one issue slot at the same FP32 rate (60 instructions
+// = 120 lanes per SM and clock, measured), which halves the issue slots of
+// arithmetic that is independent for two consecutive l.
+struct f32x2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(f32x2 x, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+}
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
+// df_factor of two l: a, g as packed (hi, lo), x broadcast with its negated hi (nxh)
+template <bool G>
+__device__ __forceinline__ void df2_factor(f32x2 ah, f32x2 al, f32x2 gh, f32x2 gl, f32x2 xh, f32x2 nxh, f32x2 xl,
+                                           dfl &t0, dfl &t1) {
+    const f32x2 np = f2_mul(ah, nxh);
+    f32x2 e = f2_fma(ah, xh, np);
+    e = f2_fma(ah, xl, e);
+    e = f2_fma(al, xh, e);
+    f32x2 h, l;
+    if (G) {
+        h = f2_sub(gh, np);
+        const f32x2 bb = f2_sub(h, gh);
+        const f32x2 err = f2_sub(f2_sub(gh, f2_sub(h, bb)), f2_add(np, bb));
+        l = f2_add(f2_add(e, gl), err);
+    } else {
+        h = f2_mul(ah, xh);
+        l = e;
+    }
+    f2_unpack(h, t0.h, t1.h);
+    f2_unpack(l, t0.l, t1.l);
 }
 
 // operators so that templated complex code (FFT butterflies) runs on dfl;

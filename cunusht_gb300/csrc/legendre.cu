@@ -29,6 +29,9 @@
 #include "kernels.cuh"
 #include "rec64.cuh"
 
+#include <algorithm>
+#include <vector>
+
 namespace cunusht {
 
 // ---------------------------------------------------------------- tables
@@ -227,18 +230,33 @@ __global__ void __launch_bounds__(LEG_TPB)
 // formed from the hi/lo parts, rounded once to FP32 and added with Kahan
 // compensation.  The start mantissa is kept in FP32 range with an exponent in
 // steps of 96 (values below 2^-56 are not accumulated).
-__global__ void k_split_coef(const double *__restrict__ c, long long n, float2 *__restrict__ out) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double v = c[i];
-    const float h = (float)v;
-    out[i] = make_float2(h, (float)(v - (double)h));
+__global__ void k_window_coef(int L, int s, const double *__restrict__ c, long long nalm, const int *__restrict__ woff,
+                              float *__restrict__ co) {
+    const int m = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int l0 = max(m, s), l = l0 + i;
+    if (i >= 128 * (woff[m + 1] - woff[m])) return;
+    float *q = co + (size_t)woff[m] * CO_WIN + (i >> 1) * 12 + (i & 1);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const dfl v = l < L ? df_from(c[k * nalm + almidx(L, m, m) - m + l]) : dfl{0.f, 0.f};
+        q[4 * k] = v.h;
+        q[4 * k + 2] = v.l;
+    }
 }
 
-int build_coef_tables_df(cunusht_plan_s *P, cudaStream_t st) {
+int build_coef_tables_df(cunusht_plan_s *P) {
+    const int L = P->lmax;
     for (int s = 0; s <= 2; ++s) {
-        const long long n = 3 * P->nalm_tab;
-        k_split_coef<<<(int)((n + 255) / 256), 256, 0, st>>>(P->d_coef[s], n, P->d_coef_df[s]);
+        std::vector<int> wo(L + 2, 0);
+        for (int m = 0; m <= L; ++m) wo[m + 1] = wo[m] + std::max(0, (L - std::max(m, s) + 128) / 128);
+        void *p = nullptr;
+        RC_TRY(plan_alloc(P, &p, wo.size() * sizeof(int)));
+        P->d_tc_woff[s] = (int *)p;
+        CU_TRY(cudaMemcpy(p, wo.data(), wo.size() * sizeof(int), cudaMemcpyHostToDevice));
+        RC_TRY(plan_alloc(P, &p, (size_t)std::max(wo[L + 1], 1) * CO_WIN * sizeof(float)));
+        P->d_tc_co[s] = (float *)p;
+        k_window_coef<<<dim3((L + 128) / 128, L + 1), 128>>>(L, s, P->d_coef[s], P->nalm_tab, P->d_tc_woff[s],
+                                                            P->d_tc_co[s]);
         CU_LAUNCH_CHECK();
     }
     return CUNUSHT_OK;
@@ -249,11 +267,11 @@ int build_coef_tables_df(cunusht_plan_s *P, cudaStream_t st) {
 template <int NB>
 __global__ void __launch_bounds__(LEG_TPB)
     k_leg_synth_s0_df(int L, const double2 *__restrict__ alm, long long astride, const double *__restrict__ lfac,
-                      const float2 *__restrict__ coef, long long nalm, const double *__restrict__ lg0,
+                      const float *__restrict__ co, const int *__restrict__ woff, const double *__restrict__ lg0,
                       int npairs, const double *__restrict__ px, const double *__restrict__ psh,
                       const double *__restrict__ pch, const int *__restrict__ prn,
                       const int *__restrict__ prs, double2 *__restrict__ H, long long hstride, int ldH) {
-    __shared__ float2 s_al[LEG_CH], s_be[LEG_CH];
+    __shared__ dfl s_al[LEG_CH], s_be[LEG_CH];
     __shared__ float4 s_a[NB][LEG_CH];
     const int m = blockIdx.y;
     const int p = blockIdx.x * LEG_TPB + threadIdx.x;
@@ -269,15 +287,15 @@ __global__ void __launch_bounds__(LEG_TPB)
     int e;
     rec_start_df(lg0[m], m, 0, sh, ch, cur, prev, e);
     kahan Er[NB], Ei[NB], Or[NB], Oi[NB];
-    const float2 *al = coef, *be = coef + 2 * nalm;
+    const float *com = co + (size_t)woff[m] * CO_WIN;
     const long long b = almidx(L, m, m) - m;
     for (int lb = m; lb <= L; lb += LEG_CH) {
         const int cnt = min(LEG_CH, L - lb + 1);
         __syncthreads();
         for (int i = threadIdx.x; i < cnt; i += LEG_TPB) {
             const long long ix = b + lb + i;
-            s_al[i] = al[ix];
-            s_be[i] = be[ix];
+            dfl gz;
+            co_load(com, lb - m + i, s_al[i], gz, s_be[i]);
             const double f = lfac ? lfac[lb + i] : 1.0;
 #pragma unroll
             for (int r = 0; r < NB; ++r) {
@@ -303,9 +321,8 @@ __global__ void __launch_bounds__(LEG_TPB)
                     }
                 }
             }
-            const float2 a2 = s_al[i], b2 = s_be[i];
-            const dfl t = df_mul_u(dfl{a2.x, a2.y}, xd);
-            const dfl nxt = df_mul_sub(t, cur, dfl{b2.x, b2.y}, prev);
+            const dfl t = df_factor<false>(s_al[i], xd, dfl{0.f, 0.f});
+            const dfl nxt = df_mul_sub(t, cur, s_be[i], prev);
             prev = cur;
             cur = nxt;
             REC_RESCALE_DF(cur, prev, e);
@@ -326,12 +343,12 @@ __global__ void __launch_bounds__(LEG_TPB)
 template <int NB>
 __global__ void __launch_bounds__(LEG_TPB)
     k_leg_synth_spin_df(int L, int spin, const double2 *__restrict__ G, const double2 *__restrict__ C,
-                        long long astride, const double *__restrict__ lfac, const float2 *__restrict__ coef,
-                        long long nalm, const double *__restrict__ lg0, int npairs, const double *__restrict__ px,
+                        long long astride, const double *__restrict__ lfac, const float *__restrict__ co,
+                        const int *__restrict__ woff, const double *__restrict__ lg0, int npairs, const double *__restrict__ px,
                         const double *__restrict__ psh, const double *__restrict__ pch,
                         const int *__restrict__ prn, const int *__restrict__ prs, double2 *__restrict__ H,
                         long long hstride, int ldH) {
-    __shared__ float2 s_al[LEG_CH], s_ga[LEG_CH], s_be[LEG_CH];
+    __shared__ dfl s_al[LEG_CH], s_ga[LEG_CH], s_be[LEG_CH];
     __shared__ float4 s_A[NB][LEG_CH], s_B[NB][LEG_CH];
     const int m = blockIdx.y;
     const int l0 = max(m, spin);
@@ -349,7 +366,7 @@ __global__ void __launch_bounds__(LEG_TPB)
     rec_start_df(lg0[m], m, spin, sh, ch, cN, pN, eN);
     rec_start_df(lg0[m], m, spin, ch, sh, cS, pS, eS);
     kahan hpn_r[NB], hpn_i[NB], hps_r[NB], hps_i[NB], hmn_r[NB], hmn_i[NB], hms_r[NB], hms_i[NB];
-    const float2 *al = coef, *ga = coef + nalm, *be = coef + 2 * nalm;
+    const float *com = co + (size_t)woff[m] * CO_WIN;
     const long long b = almidx(L, m, m) - m;
     for (int lb = l0; lb <= L; lb += LEG_CH) {
         const int cnt = min(LEG_CH, L - lb + 1);
@@ -357,9 +374,7 @@ __global__ void __launch_bounds__(LEG_TPB)
         for (int i = threadIdx.x; i < cnt; i += LEG_TPB) {
             const int l = lb + i;
             const long long ix = b + l;
-            s_al[i] = al[ix];
-            s_ga[i] = ga[ix];
-            s_be[i] = be[ix];
+            co_load(com, l - l0, s_al[i], s_ga[i], s_be[i]);
             const double f = lfac ? lfac[l] : 1.0;
             const double par = ((l + m) & 1) ? -f : f;
 #pragma unroll
@@ -390,10 +405,9 @@ __global__ void __launch_bounds__(LEG_TPB)
                     hmn_i[r].add(df_prod(B.z, B.w, cS));
                 }
             }
-            const float2 a2 = s_al[i], g2 = s_ga[i], b2 = s_be[i];
-            const dfl ad{a2.x, a2.y}, gd{g2.x, g2.y}, bd{b2.x, b2.y};
-            const dfl tN = df_fma_u(ad, xN, gd);
-            const dfl tS = df_fma_u(ad, xS, gd);
+            const dfl ad = s_al[i], gd = s_ga[i], bd = s_be[i];
+            const dfl tN = df_factor<true>(ad, xN, gd);
+            const dfl tS = df_factor<true>(ad, xS, gd);
             const dfl nN = df_mul_sub(tN, cN, bd, pN);
             const dfl nS = df_mul_sub(tS, cS, bd, pS);
             pN = cN;
@@ -701,7 +715,7 @@ __device__ __forceinline__ split2 split_c(double2 v) {
 template <int NB>
 __global__ void __launch_bounds__(LEG_TPB)
     k_leg_adj_s0_df(int L, const double2 *__restrict__ H, long long hstride, int ldH,
-                    const double *__restrict__ lfac, const float2 *__restrict__ coef, long long nalm,
+                    const double *__restrict__ lfac, const float *__restrict__ co, const int *__restrict__ woff,
                     const double *__restrict__ lg0, int npairs, const double *__restrict__ px,
                     const double *__restrict__ psh, const double *__restrict__ pch, const int *__restrict__ prn,
                     const int *__restrict__ prs, double *__restrict__ alm /* interleaved */, long long astride) {
@@ -744,7 +758,7 @@ __global__ void __launch_bounds__(LEG_TPB)
         cur.h = cur.l = 0.f;
         e = 0;
     }
-    const float2 *al = coef, *be = coef + 2 * nalm;
+    const float *com = co + (size_t)woff[m] * CO_WIN;
     const long long b = almidx(L, m, m) - m;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const dfl zero{0.f, 0.f};
@@ -755,9 +769,10 @@ __global__ void __launch_bounds__(LEG_TPB)
             const int l = lb + i;
             lam[i] = (e == 0 && l <= L) ? cur : zero;
             if (l < L) {
-                const float2 a2 = __ldg(al + b + l), b2 = __ldg(be + b + l);
-                const dfl t = df_mul_u(dfl{a2.x, a2.y}, xd);
-                const dfl nxt = df_mul_sub(t, cur, dfl{b2.x, b2.y}, prev);
+                dfl ad, gd, bd;
+                co_load(com, l - m, ad, gd, bd);
+                const dfl t = df_factor<false>(ad, xd, gd);
+                const dfl nxt = df_mul_sub(t, cur, bd, prev);
                 prev = cur;
                 cur = nxt;
                 REC_RESCALE_DF(cur, prev, e);
@@ -794,8 +809,8 @@ __global__ void __launch_bounds__(LEG_TPB)
 template <int NB>
 __global__ void __launch_bounds__(LEG_TPB)
     k_leg_adj_spin_df(int L, int spin, int ncomp, const double2 *__restrict__ H, long long hstride, int ldH,
-                      const double *__restrict__ lfac, const float2 *__restrict__ coef,
-                      long long nalm, const double *__restrict__ lg0, int npairs,
+                      const double *__restrict__ lfac, const float *__restrict__ co,
+                      const int *__restrict__ woff, const double *__restrict__ lg0, int npairs,
                       const double *__restrict__ px, const double *__restrict__ psh,
                       const double *__restrict__ pch, const int *__restrict__ prn,
                       const int *__restrict__ prs, double *__restrict__ Gout,
@@ -841,7 +856,7 @@ __global__ void __launch_bounds__(LEG_TPB)
         cN.h = cN.l = cS.h = cS.l = 0.f;
         eN = eS = 0;
     }
-    const float2 *al = coef, *ga = coef + nalm, *be = coef + 2 * nalm;
+    const float *com = co + (size_t)woff[m] * CO_WIN;
     const long long b = almidx(L, m, m) - m;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const double sgs = (spin & 1) ? -1.0 : 1.0;
@@ -854,10 +869,10 @@ __global__ void __launch_bounds__(LEG_TPB)
             lN[i] = (eN == 0 && l <= L) ? cN : zero;
             lS[i] = (eS == 0 && l <= L) ? cS : zero;
             if (l < L) {
-                const float2 a2 = __ldg(al + b + l), g2 = __ldg(ga + b + l), b2 = __ldg(be + b + l);
-                const dfl ad{a2.x, a2.y}, gd{g2.x, g2.y}, bd{b2.x, b2.y};
-                const dfl tN = df_fma_u(ad, xN, gd);
-                const dfl tS = df_fma_u(ad, xS, gd);
+                dfl ad, gd, bd;
+                co_load(com, l - l0, ad, gd, bd);
+                const dfl tN = df_factor<true>(ad, xN, gd);
+                const dfl tS = df_factor<true>(ad, xS, gd);
                 const dfl nN = df_mul_sub(tN, cN, bd, pN);
                 const dfl nS = df_mul_sub(tS, cS, bd, pS);
                 pN = cN;
@@ -1062,10 +1077,10 @@ static void launch_synth_df(const cunusht_plan_s *P, const RingPairs &R, dim3 gr
                             cudaStream_t st) {
     const int L = P->lmax;
     if (spin == 0)
-        k_leg_synth_s0_df<NB><<<grid, LEG_TPB, 0, st>>>(L, G, astride, lf, P->d_coef_df[0], P->nalm_tab, P->d_lg0[0],
+        k_leg_synth_s0_df<NB><<<grid, LEG_TPB, 0, st>>>(L, G, astride, lf, P->d_tc_co[0], P->d_tc_woff[0], P->d_lg0[0],
                                                         R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, H, hstride, R.ld);
     else
-        k_leg_synth_spin_df<NB><<<grid, LEG_TPB, 0, st>>>(L, spin, G, C, astride, lf, P->d_coef_df[spin], P->nalm_tab,
+        k_leg_synth_spin_df<NB><<<grid, LEG_TPB, 0, st>>>(L, spin, G, C, astride, lf, P->d_tc_co[spin], P->d_tc_woff[spin],
                                                           P->d_lg0[spin], R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, H,
                                                           hstride, R.ld);
 }
@@ -1103,7 +1118,7 @@ int leg_synth_batch_fl(const cunusht_plan_s *P, int nreq, int spin, const double
             CU_TRY(cudaMemsetAsync(H + r * hstride, 0, sizeof(double2) * ncols * R.ld, st));
     }
     dim3 grid((R.npairs + LEG_TPB - 1) / LEG_TPB, P->mmax + 1);
-    if (P->prec == CUNUSHT_PREC_MIXED && P->d_coef_df[spin]) {
+    if (P->prec == CUNUSHT_PREC_MIXED && P->d_tc_co[spin]) {
         for (int r0 = 0; r0 < nreq;) {
             const int left = nreq - r0;
             const double2 *Gr = G + r0 * astride, *Cr = C ? C + r0 * astride : nullptr;
@@ -1200,12 +1215,12 @@ static void launch_adj_df(const cunusht_plan_s *P, const RingPairs &R, dim3 grid
                           long long astride, cudaStream_t st) {
     const int L = P->lmax;
     if (spin == 0)
-        k_leg_adj_s0_df<NB><<<grid, LEG_TPB, 0, st>>>(L, H, hstride, R.ld, lf, P->d_coef_df[0], P->nalm_tab,
+        k_leg_adj_s0_df<NB><<<grid, LEG_TPB, 0, st>>>(L, H, hstride, R.ld, lf, P->d_tc_co[0], P->d_tc_woff[0],
                                                       P->d_lg0[0], R.npairs, R.x, R.sh, R.ch, R.rn, R.rs,
                                                       (double *)G, astride);
     else
-        k_leg_adj_spin_df<NB><<<grid, LEG_TPB, 0, st>>>(L, spin, ncomp, H, hstride, R.ld, lf, P->d_coef_df[spin],
-                                                        P->nalm_tab, P->d_lg0[spin], R.npairs, R.x, R.sh, R.ch, R.rn,
+        k_leg_adj_spin_df<NB><<<grid, LEG_TPB, 0, st>>>(L, spin, ncomp, H, hstride, R.ld, lf, P->d_tc_co[spin],
+                                                        P->d_tc_woff[spin], P->d_lg0[spin], R.npairs, R.x, R.sh, R.ch, R.rn,
                                                         R.rs, (double *)G, (double *)C, astride);
 }
 
@@ -1252,7 +1267,7 @@ int leg_adjoint_batch(const cunusht_plan_s *P, int nreq, int spin, int ncomp, co
                       void *scratch, size_t scratch_bytes) {
     const RingPairs R = pairs_of(P, cc);
     const int L = P->lmax;
-    if (P->prec == CUNUSHT_PREC_MIXED && P->use_tc && P->d_coef_df[spin] && scratch &&
+    if (P->prec == CUNUSHT_PREC_MIXED && P->use_tc && P->d_tc_co[spin] && scratch &&
         scratch_bytes >= adj_tc_scratch_bytes(P, nreq)) {
         return leg_adjoint_tc(P, nreq, spin, ncomp, H, hstride, R.ld, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.pole,
                               R.pole_rn, R.pole_rs, R.stv ? R.stv[spin] : nullptr, R.ste ? R.ste[spin] : nullptr,
@@ -1264,7 +1279,7 @@ int leg_adjoint_batch(const cunusht_plan_s *P, int nreq, int spin, int ncomp, co
     }
     dim3 grid((R.npairs + LEG_TPB - 1) / LEG_TPB, P->mmax + 1);
     const double *lf = use_lfac ? P->d_lfac : nullptr;
-    if (P->prec == CUNUSHT_PREC_MIXED && P->d_coef_df[spin]) {
+    if (P->prec == CUNUSHT_PREC_MIXED && P->d_tc_co[spin]) {
         RingPairs Rm = R;
         if (spin > 0 && R.pole == 0 && R.npairs > 1) {
             // the pole pair in closed form; the other 2^k pairs fill whole blocks

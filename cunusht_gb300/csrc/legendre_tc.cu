@@ -44,6 +44,7 @@
 #include "common.cuh"
 #include "df.cuh"
 #include "kernels.cuh"
+#include "rec64.cuh"
 #include "tcgen05.cuh"
 
 #include <algorithm>
@@ -259,7 +260,8 @@ constexpr int TCL_MIN_TAIL = 32;          // fewer leftover ring pairs than this
 // hold rings of both sides).
 template <int NB>
 struct TclLayout {
-    static constexpr int NT = NB >= 8 ? 3 : 4;           // 128-row MMA tiles per block
+    static constexpr int NT = NB >= 8 ? 3 : NB >= 4 ? 4 : 2;  // 128-row MMA tiles per block
+    static constexpr int BPS = NB >= 4 ? 1 : 2;               // blocks per SM
     static constexpr int T = 128 * NT;                   // ring threads (one ring each)
     static constexpr int BLOCK = T + 32;                 // + the MMA warp
     static constexpr int ABUF = NT * TCL_TILE;           // A buffer: NT tiles
@@ -274,13 +276,14 @@ struct TclLayout {
     // window record (written by k_tc_records, one per (m, l-window)):
     static constexpr int RSC = 4 * NO * TCL_TPS * 2;        // bf16 digit planes [4][NO][TPS], then
     static constexpr int RLS = RSC + NG * NO * 4;           // float epilogue scales [NG][NO], then
-    static constexpr int RCO = (RLS + 4 + 15) / 16 * 16;    // float lambda digit scale, then
-    static constexpr int RBE = RCO + (TCL_W + 1) * 16;      // float4 (alpha, gamma) [W + 1] and
-    static constexpr int RSZ = (RBE + (TCL_W + 1) * 8 + 15) / 16 * 16;  // float2 beta [W + 1] (zero past the window)
+    static constexpr int RSZ = (RLS + 4 + 15) / 16 * 16;    // float lambda digit scale
+    // in shared memory the window's recursion coefficients (the plan's table, co_load) follow the record
+    static constexpr int RCO = RSZ;
+    static constexpr int RBUF = RCO + CO_WIN * 4;
     static constexpr int BBUF = NN * 128;                // B' buffer: NN rows x 8 K-cores x 16 bytes
     static constexpr int OFF_B = 2 * ABUF;
     static constexpr int OFF_R = OFF_B + 2 * BBUF;       // two window records (current, next)
-    static constexpr int OFF_BAR = OFF_R + 2 * RSZ;      // full[2], empty[2], record[2]
+    static constexpr int OFF_BAR = OFF_R + 2 * RBUF;     // full[2], empty[2], record[2]
     static constexpr int OFF_TM = OFF_BAR + 48;          // tensor-memory base, give-up flag
     static constexpr int BYTES = OFF_TM + 16;
 };
@@ -310,8 +313,7 @@ __device__ __forceinline__ void tcl_pair(int pr, int &g, int &di) {
 template <int NB, bool S0>
 __global__ void __launch_bounds__(TCL_W)
     k_tc_records(int L, int spin, const double2 *__restrict__ G, const double2 *__restrict__ C, long long astride,
-                 const double *__restrict__ lfac, const float2 *__restrict__ coef, long long nalm,
-                 const int *__restrict__ woff, unsigned char *__restrict__ rec) {
+                 const double *__restrict__ lfac, const int *__restrict__ woff, unsigned char *__restrict__ rec) {
     using LY = TclLayout<NB>;
     constexpr int NO = LY::NO, NG = LY::NG;
     __shared__ float s_mx[TCL_W / 32][NO];
@@ -321,23 +323,6 @@ __global__ void __launch_bounds__(TCL_W)
     const int wb = max(m, spin) + k * TCL_W, cnt = min(TCL_W, L - wb + 1);
     unsigned char *R = rec + (size_t)(woff[m] + k) * LY::RSZ;
     const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
-    {
-        // recursion coefficients (double-float) of the window, zero past its end
-        float4 *ag = reinterpret_cast<float4 *>(R + LY::RCO);
-        float2 *bt = reinterpret_cast<float2 *>(R + LY::RBE);
-        const long long b = almidx(L, m, m) - m;
-        for (int j = i; j < TCL_W + 1; j += TCL_W) {
-            float4 a4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            float2 b2 = make_float2(0.f, 0.f);
-            if (j < cnt) {
-                const float2 a2 = coef[b + wb + j], g2 = coef[nalm + b + wb + j];
-                a4 = make_float4(a2.x, a2.y, g2.x, g2.y);
-                b2 = coef[2 * nalm + b + wb + j];
-            }
-            ag[j] = a4;
-            bt[j] = b2;
-        }
-    }
     dfl v[NO];
 #pragma unroll
     for (int o = 0; o < NO; ++o) v[o] = dfl{0.f, 0.f};
@@ -424,8 +409,9 @@ __global__ void __launch_bounds__(TCL_W)
 // side), so a block covers T pairs instead of T / 2, and the columns (E, O)
 // give theta E + O and pi - theta E - O.
 template <int NB, bool S0>
-__global__ void __launch_bounds__(TclLayout<NB>::BLOCK, 1)
-    k_leg_synth_spin_tc(int L, int spin, const unsigned char *__restrict__ rec, const int *__restrict__ woff,
+__global__ void __launch_bounds__(TclLayout<NB>::BLOCK, TclLayout<NB>::BPS)
+    k_leg_synth_spin_tc(int L, int spin, const unsigned char *__restrict__ rec, const float *__restrict__ co,
+                        const int *__restrict__ woff,
                         const double *__restrict__ lg0, int npairs,
                         const double *__restrict__ px, const double *__restrict__ psh,
                         const double *__restrict__ pch, const int *__restrict__ prn, const int *__restrict__ prs,
@@ -449,6 +435,13 @@ __global__ void __launch_bounds__(TclLayout<NB>::BLOCK, 1)
     const int m = blockIdx.y;
     const int l0 = max(m, spin);
     const unsigned char *recm = rec + (size_t)woff[m] * LY::RSZ;  // this order's window records
+    const float *com = co + (size_t)woff[m] * CO_WIN;             // and coefficients
+    auto fetch = [&](int kw, int slot) {                          // window kw into record place slot
+        const uint32_t dst = sbase + LY::OFF_R + slot * LY::RBUF, bar = rbar0 + 8 * slot;
+        mbar_expect(bar, LY::RSZ + CO_WIN * 4);
+        bulk_copy(dst, recm + (size_t)kw * LY::RSZ, LY::RSZ, bar);
+        bulk_copy(dst + LY::RCO, com + (size_t)kw * CO_WIN, CO_WIN * 4, bar);
+    };
 
     int *s_c0 = reinterpret_cast<int *>(sm + LY::OFF_TM + 8);
     if (warp == T / 32) tmem_alloc(sbase + LY::OFF_TM, LY::NCOLS);
@@ -508,7 +501,7 @@ __global__ void __launch_bounds__(TclLayout<NB>::BLOCK, 1)
     const bool work = cb < nchk;
     constexpr int CPW = TCL_W / TCL_KC;  // chunks per window
     const int kw0 = work ? cb / CPW : 0, cs0 = cb - kw0 * CPW;
-    if (tid == 0 && work) bulk_g2s(sbase + LY::OFF_R, recm + (size_t)kw0 * LY::RSZ, LY::RSZ, rbar0);
+    if (tid == 0 && work) fetch(kw0, 0);
 
     if (warp == T / 32) {
         // ---------------- MMA warp: the whole warp follows the chunk sequence (its
@@ -549,6 +542,7 @@ __global__ void __launch_bounds__(TclLayout<NB>::BLOCK, 1)
         const int tile = tid >> 7, row = tid & 127;
         const double x = act ? px[p] : 0.0;
         const dfl xd = df_from(side ? -x : x);
+        const f32x2 xh2 = f2_pack(xd.h, xd.h), nxh2 = f2_pack(-xd.h, -xd.h), xl2 = f2_pack(xd.l, xd.l);
         sum2 acc[NO];
         const uint32_t t_lane = tbase + ((uint32_t)((warp & 3) * 32) << 16) + tile * NN;  // this thread's row
         const uint32_t a_row = (uint32_t)tile * TCL_TILE + (row >> 3) * TCL_SBO + (row & 7) * 16;
@@ -562,17 +556,16 @@ __global__ void __launch_bounds__(TclLayout<NB>::BLOCK, 1)
             // finished at the previous window's closing barrier)
             if (tid == 0 && wb + TCL_W <= L) {
                 fence_async_smem();
-                bulk_g2s(sbase + LY::OFF_R + ((kl + 1) & 1) * LY::RSZ, recm + (size_t)(kw + 1) * LY::RSZ, LY::RSZ,
-                         rbar0 + 8 * ((kl + 1) & 1));
+                fetch(kw + 1, (kl + 1) & 1);
             }
             bad |= !mbar_wait(rbar0 + 8 * (kl & 1), (kl >> 1) & 1);  // this window's record has landed
-            const unsigned char *Rw = sm + LY::OFF_R + (kl & 1) * LY::RSZ;
+            const unsigned char *Rw = sm + LY::OFF_R + (kl & 1) * LY::RBUF;
             const unsigned short *s_tp = reinterpret_cast<const unsigned short *>(Rw);
             const float *s_sc = reinterpret_cast<const float *>(Rw + LY::RSC);
             const float lsc = *reinterpret_cast<const float *>(Rw + LY::RLS);
-            // recursion coefficients, zero past the window so that the steps beyond lmax stay finite
-            const float4 *s_ag = reinterpret_cast<const float4 *>(Rw + LY::RCO);
-            const float2 *s_be = reinterpret_cast<const float2 *>(Rw + LY::RBE);
+            // recursion coefficients, zero past lmax so that the steps beyond it stay finite (the alm
+            // digits there are zero)
+            const ulonglong2 *s_co = reinterpret_cast<const ulonglong2 *>(Rw + LY::RCO);
 
             const int nch = (cnt + TCL_KC - 1) / TCL_KC;
             for (int c = kw == kw0 ? cs0 : 0; c < nch; ++c, ++gc) {
@@ -604,33 +597,29 @@ __global__ void __launch_bounds__(TclLayout<NB>::BLOCK, 1)
                 // most (alpha + beta) < 2^8.5 (alpha_m ~ sqrt(2m) <= 181 for lmax <= 16383),
                 // so from below 2^40 eight steps stay below 2^108, inside the FP32
                 // range, and e (hence the digit mask) stays fixed within the half.
-                float4 agn = s_ag[c * TCL_KC];  // coefficients of the next step, loaded one step ahead
-                float2 ben = s_be[c * TCL_KC];
                 if (live) {
 #pragma unroll
                     for (int lh = 0; lh < 2; ++lh) {
                         uint32_t pk[4][4];
-                        const float scg = (act && e == 0) ? lsc : 0.f;
+                        const float scg = (act && e == 0) ? -lsc : 0.f;
+                        const f32x2 sc2 = f2_pack(scg, scg);
 #pragma unroll
                         for (int j2 = 0; j2 < 4; ++j2) {
-                            float d0[4], d1[4];
-                            // digits of lambda_l (zero unless accumulated), then one recursion step l -> l + 1
-                            auto step = [&](int i, float(&d)[4]) {
-                                digits4s(cur.h, cur.l, i < cnt ? scg : 0.f, d);
-                                const float4 ag = agn;
-                                const float2 b2 = ben;
-                                agn = s_ag[i + 1];
-                                ben = s_be[i + 1];
-                                const dfl t = df_fma_u(dfl{ag.x, ag.y}, xd, dfl{ag.z, ag.w});
-                                const dfl nxt = df_mul_sub(t, cur, dfl{b2.x, b2.y}, prev);
-                                prev = cur;
-                                cur = nxt;
-                            };
-                            const int i0 = c * TCL_KC + 8 * lh + 2 * j2;
-                            step(i0, d0);
-                            step(i0 + 1, d1);
+                            // two l at a time: the factors a x + g and the digits of both values in
+                            // packed FP32, the two recursion steps one after the other
+                            const ulonglong2 *q = s_co + 3 * (c * (TCL_KC / 2) + 4 * lh + j2);
+                            const ulonglong2 ca = q[0], cg = S0 ? ca : q[1];
+                            const float4 cb = *reinterpret_cast<const float4 *>(q + 2);
+                            dfl t0, t1;
+                            df2_factor<!S0>(f32x2{ca.x}, f32x2{ca.y}, f32x2{cg.x}, f32x2{cg.y}, xh2, nxh2, xl2, t0,
+                                            t1);
+                            const dfl v1 = df_mul_sub(t0, cur, dfl{cb.x, cb.z}, prev);
+                            uint32_t d[4];
+                            digits4x2(cur, v1, sc2, d);
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) pk[k][j2] = pack_bf16(d0[k], d1[k]);
+                            for (int k = 0; k < 4; ++k) pk[k][j2] = d[k];
+                            prev = v1;
+                            cur = df_mul_sub(t1, v1, dfl{cb.y, cb.w}, cur);
                         }
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
@@ -750,14 +739,14 @@ static int launch_synth_tc_nb(const cunusht_plan_s *P, int npairs, const double 
         return CUNUSHT_ERR_ARG;
     }
     const dim3 rgrid((L - spin + 1 + TCL_W - 1) / TCL_W, P->mmax + 1);  // m <= spin has the most windows
-    k_tc_records<NB, S0><<<rgrid, TCL_W, 0, st>>>(L, spin, G, C, astride, lf, P->d_coef_df[spin], P->nalm_tab,
-                                                  P->d_tc_woff[spin], P->d_tc_rec);
+    k_tc_records<NB, S0><<<rgrid, TCL_W, 0, st>>>(L, spin, G, C, astride, lf, P->d_tc_woff[spin], P->d_tc_rec);
     CU_LAUNCH_CHECK();
     CU_TRY(cudaFuncSetAttribute(k_leg_synth_spin_tc<NB, S0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 LY::BYTES));
     constexpr int PER = S0 ? LY::T : LY::T / 2;  // ring pairs per block
     dim3 grid((npairs + PER - 1) / PER, P->mmax + 1);
-    k_leg_synth_spin_tc<NB, S0><<<grid, LY::BLOCK, LY::BYTES, st>>>(L, spin, P->d_tc_rec, P->d_tc_woff[spin],
+    k_leg_synth_spin_tc<NB, S0><<<grid, LY::BLOCK, LY::BYTES, st>>>(L, spin, P->d_tc_rec, P->d_tc_co[spin],
+                                                                P->d_tc_woff[spin],
                                                                 P->d_lg0[spin], npairs, x, sh, ch, rn, rs, stv, ste,
                                                                 st_ld, H, hstride, ld, P->d_status);
     CU_LAUNCH_CHECK();
@@ -811,18 +800,19 @@ int tc_reserve(cunusht_plan_s *P, int nb) {
 // are.  A ring whose start is exactly zero (a pole) gets c0 = 32767 (never).
 // Entry ((m * 2 + side) * npairs + p): v = (cur.h, cur.l, prev.h, prev.l),
 // ec = (e / 96, c0); e is 0 or -96 at a ring's first chunk.
-__device__ __forceinline__ void tc_rec_step(dfl &cur, dfl &prev, dfl xd, const float2 *__restrict__ coef,
-                                            long long nalm, long long ix) {
-    const float2 a2 = coef[ix], g2 = coef[nalm + ix], b2 = coef[2 * nalm + ix];
-    const dfl t = df_fma_u(dfl{a2.x, a2.y}, xd, dfl{g2.x, g2.y});
-    const dfl nxt = df_mul_sub(t, cur, dfl{b2.x, b2.y}, prev);
+template <bool G>
+__device__ __forceinline__ void tc_rec_step(dfl &cur, dfl &prev, dfl xd, const float *__restrict__ com, int i) {
+    dfl a, g, b;
+    co_load(com, i, a, g, b);
+    const dfl nxt = df_mul_sub(df_factor<G>(a, xd, g), cur, b, prev);
     prev = cur;
     cur = nxt;
 }
 
+template <bool G>
 __global__ void k_tc_starts(int L, int spin, const double *__restrict__ lg0, int npairs, const double *__restrict__ x,
                             const double *__restrict__ sh, const double *__restrict__ ch,
-                            const float2 *__restrict__ coef, long long nalm, float4 *__restrict__ v,
+                            const float *__restrict__ co, const int *__restrict__ woff, float4 *__restrict__ v,
                             short2 *__restrict__ ec) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 2LL * npairs * (L + 1)) return;
@@ -835,7 +825,7 @@ __global__ void k_tc_starts(int L, int spin, const double *__restrict__ lg0, int
     if (side) rec_start_df(lg0[m], m, spin, ch[p], sh[p], cur, prev, e);
     else rec_start_df(lg0[m], m, spin, sh[p], ch[p], cur, prev, e);
     const dfl xd = df_from(side ? -x[p] : x[p]);
-    const long long b = almidx(L, m, m) - m;  // (l, m) at b + l
+    const float *com = co + (size_t)woff[m] * CO_WIN;
     const int nchk = l0 <= L ? (L - l0 + 1 + TCL_KC - 1) / TCL_KC : 0;
     int c = 0;
     for (; c < nchk && e != 0; ++c) {
@@ -844,14 +834,14 @@ __global__ void k_tc_starts(int L, int spin, const double *__restrict__ lg0, int
         const dfl c0 = cur, p0 = prev;
         const int e0 = e, lb = l0 + TCL_KC * c;
         for (int j = 0; j < 8; ++j)
-            if (lb + j <= L) tc_rec_step(cur, prev, xd, coef, nalm, b + lb + j);
+            if (lb + j <= L) tc_rec_step<G>(cur, prev, xd, com, lb - l0 + j);
         REC_RESCALE_DF(cur, prev, e);
         if (e == 0) {
             cur = c0, prev = p0, e = e0;
             break;
         }
         for (int j = 8; j < TCL_KC; ++j)
-            if (lb + j <= L) tc_rec_step(cur, prev, xd, coef, nalm, b + lb + j);
+            if (lb + j <= L) tc_rec_step<G>(cur, prev, xd, com, lb - l0 + j);
         REC_RESCALE_DF(cur, prev, e);
     }
     const bool never = c >= nchk || (cur.h == 0.f && prev.h == 0.f);
@@ -890,8 +880,12 @@ int tc_start_states(cunusht_plan_s *P, int g, int s, bool enable) {
         CU_TRY(e);
     }
     P->ws_bytes += bytes;
-    k_tc_starts<<<(unsigned)((n + 255) / 256), 256>>>(L, s, P->d_lg0[s], np, x, sh, ch, P->d_coef_df[s],
-                                                     P->nalm_tab, P->d_tc_stv[g][s], P->d_tc_ste[g][s]);
+    auto build = [&](auto kern) {
+        kern<<<(unsigned)((n + 255) / 256), 256>>>(L, s, P->d_lg0[s], np, x, sh, ch, P->d_tc_co[s], P->d_tc_woff[s],
+                                                   P->d_tc_stv[g][s], P->d_tc_ste[g][s]);
+    };
+    if (s == 0) build(k_tc_starts<false>);
+    else build(k_tc_starts<true>);
     CU_LAUNCH_CHECK();
     CU_TRY(cudaDeviceSynchronize());  // the tables are read from any stream
     return CUNUSHT_OK;
@@ -906,12 +900,9 @@ int tc_plan_init(cunusht_plan_s *P) {
     }
     size_t nrec = 0;
     for (int s = 0; s <= 2 && s <= L; ++s) {
-        std::vector<int> wo(L + 2, 0);
-        for (int m = 0; m <= L; ++m) wo[m + 1] = wo[m] + (L - std::max(m, s) + 1 + TCL_W - 1) / TCL_W;
-        CU_TRY(cudaMalloc(&P->d_tc_woff[s], wo.size() * sizeof(int)));
-        CU_TRY(cudaMemcpy(P->d_tc_woff[s], wo.data(), wo.size() * sizeof(int), cudaMemcpyHostToDevice));
-        P->ws_bytes += wo.size() * sizeof(int);
-        nrec = std::max(nrec, (size_t)wo[L + 1]);
+        size_t w = 0;
+        for (int m = 0; m <= L; ++m) w += (L - std::max(m, s) + TCL_W) / TCL_W;
+        nrec = std::max(nrec, w);
     }
     P->tc_nrec = nrec;
     return tc_reserve(P, 1);  // single requests; cunusht_plan_reserve_batch grows it
@@ -1054,7 +1045,7 @@ int leg_synth_spin_tc(const cunusht_plan_s *P, int nb, int npairs, const double 
         if (stv) ++stv, ++ste;
         --npairs;
     }
-    const int per = (nb == 8 ? TclLayout<8>::T : TclLayout<4>::T) / (spin == 0 ? 1 : 2), tail = npairs % per;
+    const int per = (nb == 8 ? TclLayout<8>::T : 512) / (spin == 0 ? 1 : 2), tail = npairs % per;
     const int ntc = (npairs > per && tail < TCL_MIN_TAIL) ? npairs - tail : npairs;
     auto launch = [&](auto nbc) {
         constexpr int NBV = decltype(nbc)::value;

@@ -12,8 +12,8 @@
 //   * mu and the alm are split into seven 8-bit digits on the integer pipe
 //     (rec64.cuh) and multiplied on the tensor cores,
 //         mu = 2^El 2^-7 sum_i d_i 2^-8i,   c a = 2^Ea 2^-7 sum_j t_j 2^-8j,
-//     El per l-window from the bound sqrt((2l + 1) / (4 pi)) / c_l, Ea per
-//     window and column from the largest |c a|.  The digits are exact in fp16,
+//     El per 16 l from the bound sqrt((2l + 1) / (4 pi)) / c_l, Ea per window
+//     and column from the largest |c a|.  The digits are exact in fp16,
 //     their products of equal weight g = i + j <= 6 (28 of the 49 pairs, the
 //     rest below 2^-56) are summed over 128 l in FP32 tensor memory: at most
 //     7 x 128 products below 2^14, an integer below 2^24, so no rounding
@@ -59,10 +59,10 @@ constexpr int T6_ABUF = T6_NT * T6_TILE;
 constexpr int T6_BBUF = T6_NN * 128;
 constexpr int T6_TPS = T6_W + 8;          // digit-plane row stride (elements)
 // window record: fp16 digit planes [7][4][TPS], double epilogue scales [2][4],
-// lambda exponent, double2 (a, g) [W + 1] (zero past the window)
+// mu exponents per 16 l, double2 (a, g) [W + 1] (zero past the window)
 constexpr int T6_RSC = T6_ND * T6_NO * T6_TPS * 2;
 constexpr int T6_REL = T6_RSC + 2 * T6_NO * 8;
-constexpr int T6_RCO = T6_REL + 16;
+constexpr int T6_RCO = T6_REL + 32;
 constexpr int T6_RSZ = T6_RCO + (T6_W + 1) * 16;
 constexpr int T6_OFF_B = 2 * T6_ABUF;
 constexpr int T6_OFF_R = T6_OFF_B + 2 * T6_BBUF;
@@ -150,13 +150,6 @@ __global__ void k_tc64_coef(int L, int s, const double2 *__restrict__ c, double2
     cl[ix] = c[ix].x;
 }
 
-// 2^El > |mu_l| for the l of [lb, lhi]: from sqrt((2l + 1) / (4 pi)) / c_l
-__device__ __forceinline__ int tc64_bound_exp(double c, int l) {
-    int e;
-    frexpf(1.0001f * sqrtf((2.f * l + 1.f) * 0.0795774715459476679f) / (float)c, &e);
-    return e;
-}
-
 // El of every chunk of 16 l (from l0) of every order: entry 8 woff[m] + chunk
 __global__ void k_tc64_chunk_exp(int L, int s, const double *__restrict__ cl, const int *__restrict__ woff,
                                  short *__restrict__ eb) {
@@ -165,7 +158,7 @@ __global__ void k_tc64_chunk_exp(int L, int s, const double *__restrict__ cl, co
     if (lb > L) return;
     const long long b = almidx(L, m, m) - m;
     int e = -1000;
-    for (int l = lb; l <= min(lb + 15, L); ++l) e = max(e, tc64_bound_exp(cl[b + l], l));
+    for (int l = lb; l <= min(lb + 15, L); ++l) e = max(e, tc_bound_exp((float)cl[b + l], l));
     eb[8 * (long long)woff[m] + c] = (short)e;
 }
 
@@ -219,16 +212,15 @@ __global__ void k_tc64_starts(int L, int spin, const double2 *__restrict__ lg0, 
 // ---------------------------------------------------------------- window records
 // One block of 128 threads per (window k, order m), thread i for l = wb + i:
 // the four alm combinations of legendre.cu times c_l, their column exponents
-// and digit planes, the epilogue scales 2^(El + Ea - 14 - 24) and 2^(El + Ea -
-// 14 - 48) (NaN when the window's column holds a non-finite value, so that it
-// reaches every ring of the order), the lambda exponent and the window's
+// and digit planes, the epilogue scales 2^(Ea - 14 - 24) and 2^(Ea - 14 - 48) (NaN when the window's column holds a non-finite value, so that it
+// reaches every ring of the order), the mu exponents and the window's
 // recursion coefficients.  Spin 0: the columns are the alm split by the parity
 // of l + m, (E re, E im, O re, O im).
 __global__ void __launch_bounds__(T6_W)
     k_tc64_records(int L, int spin, const double2 *__restrict__ G, const double2 *__restrict__ C,
                    const double *__restrict__ lfac, const double2 *__restrict__ ag, const double *__restrict__ cl,
                    const int *__restrict__ woff, unsigned char *__restrict__ rec) {
-    __shared__ int s_mx[T6_W / 32][T6_NO + 1];
+    __shared__ int s_mx[T6_W / 32][T6_NO];
     __shared__ int s_ea[T6_NO];
     const int m = blockIdx.y, k = blockIdx.x;
     if (k >= woff[m + 1] - woff[m]) return;
@@ -246,7 +238,7 @@ __global__ void __launch_bounds__(T6_W)
         const double c = cl[ix], f = (lfac ? lfac[l] : 1.0) * c;
         const bool odd = (l + m) & 1;
         const double2 g = G[ix];
-        eb = tc64_bound_exp(c, l);
+        eb = tc_bound_exp((float)c, l);
         if (spin == 0) {
             v[odd ? 2 : 0] = f * g.x;
             v[odd ? 3 : 1] = f * g.y;
@@ -259,27 +251,28 @@ __global__ void __launch_bounds__(T6_W)
             v[3] = par * (cc.x - g.y);
         }
     }
+    // digit exponent of mu over the chunk of 16 l, 2^El > |mu_l|; the alm take the factor 2^El, so
+    // that c_l, which falls by a factor 3 over the first l of an order, costs no digit
+#pragma unroll
+    for (int sft = 8; sft > 0; sft >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, sft));
+    if (i % 16 == 0) reinterpret_cast<int *>(R + T6_REL)[i / 16] = eb;
 #pragma unroll
     for (int o = 0; o < T6_NO; ++o) {
+        if (i < cnt) v[o] = scalbn(v[o], eb);
         const int ex = __reduce_max_sync(0xffffffffu, (__double2hiint(v[o]) >> 20) & 0x7FF);
         if (lane == 0) s_mx[warp][o] = ex;
     }
-    {
-        const int ex = __reduce_max_sync(0xffffffffu, eb);
-        if (lane == 0) s_mx[warp][T6_NO] = ex;
-    }
     __syncthreads();
     if (i < T6_NO) {
-        int ex = 0, el = -1000;
+        int ex = 0;
 #pragma unroll
-        for (int w = 0; w < T6_W / 32; ++w) ex = max(ex, s_mx[w][i]), el = max(el, s_mx[w][T6_NO]);
+        for (int w = 0; w < T6_W / 32; ++w) ex = max(ex, s_mx[w][i]);
         double *sc = reinterpret_cast<double *>(R + T6_RSC);
         const int ea = max(ex, 64) - 1022;  // 2^ea > |v| (zero columns: digits 0)
         const bool bad = ex == 0x7FF;
         s_ea[i] = ea;
-        sc[i] = bad ? nan("") : scalbn(1.0, el + ea - 14 - 24);
-        sc[T6_NO + i] = bad ? nan("") : scalbn(1.0, el + ea - 14 - 48);
-        if (i == 0) *reinterpret_cast<int *>(R + T6_REL) = el;
+        sc[i] = bad ? nan("") : scalbn(1.0, ea - 14 - 24);
+        sc[T6_NO + i] = bad ? nan("") : scalbn(1.0, ea - 14 - 48);
     }
     __syncthreads();
     unsigned short *tp = reinterpret_cast<unsigned short *>(R);
@@ -432,7 +425,7 @@ __global__ void __launch_bounds__(T6_BLOCK, 1)
             const unsigned char *Rw = sm + T6_OFF_R + (kl & 1) * T6_RSZ;
             const unsigned short *s_tp = reinterpret_cast<const unsigned short *>(Rw);
             const double *s_sc = reinterpret_cast<const double *>(Rw + T6_RSC);
-            const int nb0 = 1030 + *reinterpret_cast<const int *>(Rw + T6_REL);
+            const int *s_el = reinterpret_cast<const int *>(Rw + T6_REL);
             const double2 *s_ag = reinterpret_cast<const double2 *>(Rw + T6_RCO);
 
             const int nch = (cnt + T6_KC - 1) / T6_KC;
@@ -446,7 +439,7 @@ __global__ void __launch_bounds__(T6_BLOCK, 1)
                     *reinterpret_cast<uint4 *>(sB + b_dst) =
                         *reinterpret_cast<const uint4 *>(s_tp + b_src + c * T6_KC);
                 if (live) {
-                    const int nb = nb0 - e;  // e < 0: every digit 0
+                    const int nb = 1030 + s_el[c >> 1] - e;  // e < 0: every digit 0
                     uint32_t pk[T6_ND][4];
 #pragma unroll
                     for (int j2 = 0; j2 < 4; ++j2) {

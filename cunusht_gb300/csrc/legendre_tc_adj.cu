@@ -39,6 +39,7 @@
 #include "common.cuh"
 #include "df.cuh"
 #include "kernels.cuh"
+#include "rec64.cuh"
 #include "tcgen05.cuh"
 
 namespace cunusht {
@@ -122,7 +123,8 @@ __global__ void k_adj_hmax(const double2 *__restrict__ H, long long hstride, int
 template <int NB, bool S0>
 __global__ void __launch_bounds__(TCA_THREADS, 1)
     k_leg_adj_tc(int L, int spin, const double2 *__restrict__ H, long long hstride, int ldH,
-                 const float2 *__restrict__ coef, long long nalm, const double *__restrict__ lg0, int npairs,
+                 const float *__restrict__ co, const int *__restrict__ woff, long long nalm,
+                 const double *__restrict__ lg0, int npairs,
                  const double *__restrict__ px, const double *__restrict__ psh, const double *__restrict__ pch,
                  const int *__restrict__ prn, const int *__restrict__ prs, const float4 *__restrict__ stv,
                  const short2 *__restrict__ ste, int st_ld, const float *__restrict__ hm, int npairs_all,
@@ -352,7 +354,9 @@ __global__ void __launch_bounds__(TCA_THREADS, 1)
         // ---------------- ring warps
         const double x = act ? px[p] : 0.0;
         const dfl xd = df_from(side ? -x : x);
-        const float2 *al = coef, *ga = coef + nalm, *be = coef + 2 * nalm;
+        const f32x2 xh2 = f2_pack(xd.h, xd.h), nxh2 = f2_pack(-xd.h, -xd.h), xl2 = f2_pack(xd.l, xd.l);
+        // coefficients, zero past lmax (the values there stay finite and are not used)
+        const ulonglong2 *com = reinterpret_cast<const ulonglong2 *>(co + (size_t)woff[m] * CO_WIN);
         const uint32_t boff = (tid >> 3) * TCA_B_LBO + (tid & 7) * 16;
         int gc = 0, bad = 0;
         for (int lb = lstart; lb <= L; lb += TCA_KC, ++gc) {
@@ -370,28 +374,22 @@ __global__ void __launch_bounds__(TCA_THREADS, 1)
 #pragma unroll
                 for (int lh = 0; lh < 2; ++lh) {
                     uint32_t pk[4][4];
-                    const float scg = (act && e == 0) ? lsc : 0.f;
+                    const float scg = (act && e == 0) ? -lsc : 0.f;
+                    const f32x2 sc2 = f2_pack(scg, scg);
 #pragma unroll
-                    for (int j2 = 0; j2 < 4; ++j2) {
-                        float d0[4], d1[4];
-                        auto step = [&](int l, float(&d)[4]) {
-                            digits4s(cur.h, cur.l, l <= L ? scg : 0.f, d);
-                            float2 a2 = make_float2(0.f, 0.f), g2 = a2, b2 = a2;
-                            if (l < L) {
-                                a2 = __ldg(al + b + l);
-                                g2 = __ldg(ga + b + l);
-                                b2 = __ldg(be + b + l);
-                            }
-                            const dfl t = df_fma_u(dfl{a2.x, a2.y}, xd, dfl{g2.x, g2.y});
-                            const dfl nxt = df_mul_sub(t, cur, dfl{b2.x, b2.y}, prev);
-                            prev = cur;
-                            cur = nxt;
-                        };
-                        const int l = lb + 8 * lh + 2 * j2;
-                        step(l, d0);
-                        step(l + 1, d1);
+                    for (int j2 = 0; j2 < 4; ++j2) {  // two l at a time, as in the synthesis
+                        const ulonglong2 *q = com + 3 * ((lb - l0) / 2 + 4 * lh + j2);
+                        const ulonglong2 ca = __ldg(q), cg = S0 ? ca : __ldg(q + 1);
+                        const float4 cb = __ldg(reinterpret_cast<const float4 *>(q + 2));
+                        dfl t0, t1;
+                        df2_factor<!S0>(f32x2{ca.x}, f32x2{ca.y}, f32x2{cg.x}, f32x2{cg.y}, xh2, nxh2, xl2, t0, t1);
+                        const dfl v1 = df_mul_sub(t0, cur, dfl{cb.x, cb.z}, prev);
+                        uint32_t d[4];
+                        digits4x2(cur, v1, sc2, d);
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) pk[k][j2] = pack_bf16(d0[k], d1[k]);
+                        for (int k = 0; k < 4; ++k) pk[k][j2] = d[k];
+                        prev = v1;
+                        cur = df_mul_sub(t1, v1, dfl{cb.y, cb.w}, cur);
                     }
 #pragma unroll
                     for (int k = 0; k < 4; ++k)  // digit k of lambda -> N-core (k, lh)
@@ -519,7 +517,8 @@ static int launch_adj_tc_nb(const cunusht_plan_s *P, const TcAdjArgs &A, int r0,
     constexpr int PER = S0 ? TCA_R : TCA_R / 2;
     const dim3 grid((A.ntc + PER - 1) / PER, P->mmax + 1);
     k_leg_adj_tc<NB, S0><<<grid, TCA_THREADS, TCA_BYTES, st>>>(
-        P->lmax, A.spin, A.H + r0 * A.hstride, A.hstride, A.ld, P->d_coef_df[A.spin], P->nalm_tab, P->d_lg0[A.spin],
+        P->lmax, A.spin, A.H + r0 * A.hstride, A.hstride, A.ld, P->d_tc_co[A.spin], P->d_tc_woff[A.spin],
+        P->nalm_tab, P->d_lg0[A.spin],
         A.ntc, A.x, A.sh, A.ch, A.rn, A.rs, A.stv, A.ste, A.st_ld, A.hm + r0, A.npairs_all,
         A.acc + (long long)r0 * P->nalm_tab * 4, P->d_status);
     CU_LAUNCH_CHECK();

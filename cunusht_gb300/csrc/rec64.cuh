@@ -102,6 +102,25 @@ __device__ __forceinline__ void tc64_start(double2 lg0, int m, int s, RingLog q,
     else rec_start_dd(lg0, m, s, a, b, isinf(a.x), isinf(b.x), cur, prev, e);
 }
 
+// Coefficients alpha_l, gamma_l, beta_l of the double-float recursion of the
+// mixed plans, laid out for the packed steps: windows of 128 l from l0 = max(m,
+// s), window k of order m at woff[m] + k, twelve floats per pair of l (a_l.h,
+// a_{l+1}.h, a_l.l, a_{l+1}.l, then gamma, then beta), zero from l = L on.
+constexpr int CO_WIN = 64 * 12;  // floats per window
+__device__ __forceinline__ void co_load(const float *__restrict__ com, int i, dfl &a, dfl &g, dfl &b) {
+    const float *q = com + (i >> 1) * 12 + (i & 1);  // i = l - l0, com: the order's first window
+    a = dfl{q[0], q[2]};
+    g = dfl{q[4], q[6]};
+    b = dfl{q[8], q[10]};
+}
+
+// 2^El > |mu_l| from the bound sqrt((2l + 1) / (4 pi)) / c_l
+__device__ __forceinline__ int tc_bound_exp(float c, int l) {
+    int e;
+    frexpf(1.0001f * sqrtf((2.f * l + 1.f) * 0.0795774715459476679f) / c, &e);
+    return e;
+}
+
 // ---------------------------------------------------------------- digits
 // v = 2^Eb 2^-7 sum_{i<7} d_i 2^-8i with integer digits |d_i| <= 128: the
 // fixed-point value X = v 2^(55 - Eb) (truncated; |v| < 2^Eb, so |X| <= 2^55)

@@ -4,6 +4,8 @@
 #pragma once
 #include <cstdint>
 
+#include "df.cuh"
+
 namespace cunusht {
 
 // ---------------------------------------------------------------- tcgen05 / mbarrier helpers
@@ -82,6 +84,16 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // (both addresses 16-byte aligned, bytes a multiple of 16)
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// the two halves of bulk_g2s: several copies counted as one phase
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
@@ -171,6 +183,24 @@ __device__ __forceinline__ void digits4s(float h, float l, float sc, float (&d)[
     for (int k = 1; k < 4; ++k) {
         d[k] = __fsub_rn(__fmaf_rn(r, 256.f, RND), RND);
         r = __fmaf_rn(r, 256.f, -d[k]);
+    }
+}
+
+// digits4s of two values v0, v1 in packed FP32 (the same digits), each digit
+// pair as packed bf16 (v0 low); sc2: the broadcast scale, negated
+__device__ __forceinline__ void digits4x2(dfl v0, dfl v1, f32x2 sc2, uint32_t (&d)[4]) {
+    const f32x2 rnd = f2_pack(12582912.f, 12582912.f), c256 = f2_pack(256.f, 256.f);
+    const f32x2 h = f2_pack(v0.h, v1.h), l = f2_pack(v0.l, v1.l);
+    f32x2 q = f2_sub(rnd, f2_fma(h, sc2, rnd));  // the digit: minus the rounded negated value
+    f32x2 r = f2_fma(l, sc2, f2_fma(h, sc2, q));
+    float a, b;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        f2_unpack(q, a, b);
+        d[k] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+        if (k == 3) break;
+        q = f2_sub(rnd, f2_fma(r, c256, rnd));
+        r = f2_fma(r, c256, q);
     }
 }
 
