@@ -122,7 +122,7 @@ template <typename T> static int upload(cunusht_plan_s *P, T **p, const std::vec
 
 static void free_plan(cunusht_plan_s *P) {
     if (!P) return;
-    void *ptrs[] = {P->d_ring_sc, P->d_ring_theta, P->d_ring_phi0, P->d_ring_nph, P->d_ring_ofs, P->d_gl_x, P->d_gl_sh,
+    void *ptrs[] = {P->d_ring_sc, P->d_ring_geo, P->d_ring_theta, P->d_ring_phi0, P->d_ring_nph, P->d_ring_ofs, P->d_gl_x, P->d_gl_sh,
                     P->d_gl_ch, P->d_gl_rn, P->d_gl_rs, P->d_cc_x, P->d_cc_sh, P->d_cc_ch, P->d_cc_rn,
                     P->d_cc_rs, P->d_Dth, P->d_Dph, P->d_coef[0], P->d_coef[1], P->d_coef[2], P->d_lg0[0],
                     P->d_lg0[1], P->d_lg0[2], P->d_lfac, P->d_tc_co[0], P->d_tc_co[1], P->d_tc_co[2], P->d_tw64, P->d_tw32, P->d_twdf, P->d_chirp_df, P->d_bker_df, P->d_chirp, P->d_bker,
@@ -275,6 +275,14 @@ static int build_plan(cunusht_plan_s *P, int lmax, double eps, int precision, in
             sc[i] = make_float4(s_.h, s_.l, c_.h, c_.l);
         }
         RC_TRY(upload(P, &P->d_ring_sc, sc));
+        if (P->prec == CUNUSHT_PREC_FP64) {
+            std::vector<RingGeo> geo(nring);
+            for (int i = 0; i < nring; ++i) {
+                const double s_ = std::sin(P->h_theta[i]), c_ = std::cos(P->h_theta[i]);
+                geo[i] = RingGeo{s_, c_, c_ / s_, TWOPI / (double)P->h_nph[i]};
+            }
+            RC_TRY(upload(P, &P->d_ring_geo, geo));
+        }
     }
 
     // ---- torus and fine grid
@@ -955,7 +963,7 @@ int cunusht_dlm2pointing(cunusht_plan_t *P, const void *dlm, const void *dclm, i
                                          P->d_ring_ofs, P->npix, P->d_glmap, P->d_glmap + P->npix, ptg,
                                          ptg + P->npix, gamma, st));
         else
-            RC_TRY(pointing_launch(P->nring, P->d_ring_theta, P->d_ring_phi0, P->d_ring_nph, P->d_ring_ofs,
+            RC_TRY(pointing_launch(P->nring, P->nph_uniform, P->d_ring_geo, P->d_ring_theta, P->d_ring_phi0, P->d_ring_nph, P->d_ring_ofs,
                                    P->npix, P->d_glmap, P->d_glmap + P->npix, ptg, ptg + P->npix, gamma, st));
     }
     return CUNUSHT_OK;
@@ -1037,7 +1045,7 @@ int cunusht_lensing_vjp_dlm(cunusht_plan_t *P, int spin, const void *gclm, int a
     }
     RC_TRY(leg_synth(P, 1, D, nullptr, true, false, P->d_Hgl, st));
     RC_TRY(ring_synth(P, 1, P->d_Hgl, P->d_glmap, P->d_glmap + P->npix, st));
-    RC_TRY(pointing_launch(P->nring, P->d_ring_theta, P->d_ring_phi0, P->d_ring_nph, P->d_ring_ofs, P->npix,
+    RC_TRY(pointing_launch(P->nring, P->nph_uniform, P->d_ring_geo, P->d_ring_theta, P->d_ring_phi0, P->d_ring_nph, P->d_ring_ofs, P->npix,
                            P->d_glmap, P->d_glmap + P->npix, ptg, ptg + P->npix, nullptr, st));
     // fine grid of the unlensed field
     const double2 *G = (const double2 *)gclm;
@@ -1117,7 +1125,7 @@ int cunusht_pointing(int nring, const double *ring_theta, const double *ring_phi
     ARG_CHECK(nring >= 1 && ring_theta && ring_phi0 && ring_nph && ring_ofs, "ring tables missing");
     ARG_CHECK(s1t && s1p && ot && op, "NULL array argument");
     ARG_CHECK(npix >= 0, "npix must be >= 0");
-    return pointing_launch(nring, ring_theta, ring_phi0, (const long long *)ring_nph, (const long long *)ring_ofs,
+    return pointing_launch(nring, 0, nullptr, ring_theta, ring_phi0, (const long long *)ring_nph, (const long long *)ring_ofs,
                            npix, s1t, s1p, ot, op, og, (cudaStream_t)stream);
 }
 

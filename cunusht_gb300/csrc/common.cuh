@@ -151,6 +151,11 @@ constexpr int MR_NMAX = 8192;
 constexpr int MR_MAXST = 16;
 constexpr int MR_KMAX = 128;
 
+// sin, cos and cot of a ring's colatitude, pixel spacing 2 pi / nph
+struct RingGeo {
+    double st, ct, cot, dphi;
+};
+
 // log2 sin(theta/2) and log2 cos(theta/2) of a ring as FP64 pairs (high part -inf for a zero)
 struct RingLog {
     double sh, sl, ch, cl;
@@ -177,6 +182,7 @@ struct cunusht_plan_s {
     std::vector<long long> h_nph, h_ofs;
     double *d_ring_theta = nullptr, *d_ring_phi0 = nullptr;
     long long *d_ring_nph = nullptr, *d_ring_ofs = nullptr;
+    RingGeo *d_ring_geo = nullptr;
     float4 *d_ring_sc = nullptr;  // (sin theta, cos theta) per ring as hi/lo FP32 pairs
     // ring pairs (theta, pi - theta) of the pointing geometry
     int gl_npairs = 0;

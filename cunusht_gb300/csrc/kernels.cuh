@@ -143,8 +143,8 @@ int nufft_spread(const cunusht_plan_s *P, int spin, const double *loc, long long
                  cudaStream_t st);
 
 // pointing.cu
-int pointing_launch(int nring, const double *rth, const double *rph0, const long long *rnph,
-                    const long long *rofs, long long npix, const double *dth, const double *dph,
+int pointing_launch(int nring, int nph_uniform, const RingGeo *geo, const double *rth, const double *rph0,
+                    const long long *rnph, const long long *rofs, long long npix, const double *dth, const double *dph,
                     double *out_th, double *out_ph, double *out_gamma, cudaStream_t st);
 int pointing_mixed_launch(int nring, int nph_uniform, const double *rth, const float4 *rsc, const double *rph0,
                           const long long *rnph, const long long *rofs, long long npix, const double *dth,

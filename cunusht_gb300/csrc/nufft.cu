@@ -19,15 +19,42 @@
 
 namespace cunusht {
 
-template <typename T, int W = MAXW>
-__device__ __forceinline__ void weights(const PointCoords &pc, int w, T beta, T *kt, T *kp) {
-    const T s = (T)2 / (T)w;
+// One weight, out of line: 2 W copies in each of the 30 kernels below would triple the compile time
+// (a call costs about a tenth of the 110 instructions it makes).
+static __device__ __noinline__ double es_weight64(dfl f0, float a, dfl s, dfl nbeta, const float2 *T) {
+    return df_to(es_kernel_df<false>(f0, a, EsParams{s, nbeta}, T, nullptr));
+}
+
+// FP64 kernel weights of the W taps per axis: the split evaluation up to
+// ES_SPLIT_MAXW taps, FP64 exp and sqrt above
+template <int W>
+__device__ __forceinline__ void weights64(const PointCoords &pc, double beta, const float2 *T, double *kt, double *kp) {
+    if constexpr (W <= ES_SPLIT_MAXW) {
+        const EsParams E{df_from(2.0 / W), df_from(-beta)};
+        const dfl ft = df_from(pc.ft), fp = df_from(pc.fp);
 #pragma unroll
-    for (int a = 0; a < W; ++a) {
-        if (W < MAXW || a < w) {  // exact trip count when the width is a template argument
-            kt[a] = es_kernel<T>(((T)pc.ft + (T)a) * s, beta);
-            kp[a] = es_kernel<T>(((T)pc.fp + (T)a) * s, beta);
+        for (int a = 0; a < W; ++a) {
+            kt[a] = es_weight64(ft, (float)a, E.s, E.nbeta, T);
+            kp[a] = es_weight64(fp, (float)a, E.s, E.nbeta, T);
         }
+    } else {
+        const double s = 2.0 / W;
+#pragma unroll
+        for (int a = 0; a < W; ++a) {
+            kt[a] = es_kernel<double>((pc.ft + a) * s, beta);
+            kp[a] = es_kernel<double>((pc.fp + a) * s, beta);
+        }
+    }
+}
+
+// e^{i x}: the series below 1/16 (error below 1e-18), where the rotation angles lie away from the poles
+__device__ __forceinline__ void sincos_small(double x, double &s, double &c) {
+    if (fabs(x) < 0.0625) {
+        const double x2 = x * x;
+        s = x + x * x2 * (-1.0 / 6.0 + x2 * (1.0 / 120.0 + x2 * (-1.0 / 5040.0 + x2 * (1.0 / 362880.0 - x2 * (1.0 / 39916800.0)))));
+        c = 1.0 + x2 * (-0.5 + x2 * (1.0 / 24.0 + x2 * (-1.0 / 720.0 + x2 * (1.0 / 40320.0 - x2 * (1.0 / 3628800.0)))));
+    } else {
+        sincos(x, &s, &c);
     }
 }
 
@@ -42,12 +69,21 @@ template <int W0 = 2, typename F> static void with_width(int w, F &&f) {
 }
 
 // ------------------------------------------------------------ interp (type 2)
-template <typename T, bool CPLX, int W>
+// FP64 plans.  With the split weights the w^2 (2 w^2 complex) products on the FP64 pipe bound it:
+// lmax 2047 spin 2, w 9, 8.4 M points 11.9 -> 3.9 ms (FP64 exp and sqrt were 600 of 850 FP64 instructions
+// per point; about 270 are left).
+template <bool CPLX, int W>
 __global__ void __launch_bounds__(NU_TPB)
-    k_interp(const T *__restrict__ U, int nrows, int Npf, int Ntf, int n_lo, int w, T beta,
+    k_interp(const double *__restrict__ U, int nrows, int Npf, int Ntf, int n_lo, double beta,
              const double *__restrict__ loc, long long npts, int layout,
              const double *__restrict__ gamma, int spin, void *__restrict__ out, int out_f32, long long ubs,
              long long lbs, long long obs) {
+    using T = double;
+    __shared__ float2 s_exp2[128];
+    if (W <= ES_SPLIT_MAXW) {
+        if (threadIdx.x < 128) s_exp2[threadIdx.x] = ES_EXP2[threadIdx.x];
+        __syncthreads();
+    }
     const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= npts) return;
     U += blockIdx.y * ubs;  // request of a batch (strides in elements)
@@ -58,7 +94,7 @@ __global__ void __launch_bounds__(NU_TPB)
     load_point(loc, j, npts, layout, th, ph);
     const PointCoords pc = point_coords(th, ph, Ntf, Npf, n_lo, nrows, W);
     T kt[W], kp[W];
-    weights<T, W>(pc, W, beta, kt, kp);
+    weights64<W>(pc, beta, s_exp2, kt, kp);
     int cols[W];
 #pragma unroll
     for (int b = 0; b < W; ++b) {
@@ -91,7 +127,7 @@ __global__ void __launch_bounds__(NU_TPB)
         double zr = ar, zi = ai;
         if (gamma) {
             double s, c;
-            sincos(spin * gamma[j], &s, &c);
+            sincos_small(spin * gamma[j], s, c);
             const double tr = zr * c - zi * s;
             zi = zr * s + zi * c;
             zr = tr;
@@ -121,13 +157,19 @@ __global__ void __launch_bounds__(NU_TPB)
 // points) add their taps to U directly.
 constexpr int SPW_WARPS = 4;  // warps per block
 
-template <typename T, bool CPLX, int W>
+template <bool CPLX, int W>
 __global__ void __launch_bounds__(SPW_WARPS * 32)
-    k_spread_warp(T *__restrict__ U, int nrows, int Npf, int Ntf, int n_lo, int w, T beta,
+    k_spread_warp(double *__restrict__ U, int nrows, int Npf, int Ntf, int n_lo, double beta,
                   const double *__restrict__ loc, long long npts, int layout, const double *__restrict__ gamma,
                   int spin, const void *__restrict__ in, int in_f32, int SR, int SC, long long ubs, long long lbs,
                   long long ibs, unsigned long long *__restrict__ Ufix, const float *__restrict__ vmax, int lgn) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    using T = double;
+    __shared__ float2 s_exp2[128];
+    if (W <= ES_SPLIT_MAXW) {
+        if (threadIdx.x < 128) s_exp2[threadIdx.x] = ES_EXP2[threadIdx.x];
+        __syncthreads();
+    }
     constexpr int NC = CPLX ? 2 : 1;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     T *strip = reinterpret_cast<T *>(smem_raw) + (size_t)wid * SR * SC * NC;
@@ -157,14 +199,14 @@ __global__ void __launch_bounds__(SPW_WARPS * 32)
         }
         if (CPLX && gamma) {
             double s, c;
-            sincos(spin * gamma[j], &s, &c);  // multiply by e^{-i spin gamma}
+            sincos_small(spin * gamma[j], s, c);  // multiply by e^{-i spin gamma}
             const double t2 = vr * c + vi * s;
             vi = vi * c - vr * s;
             vr = t2;
         }
     }
     T kt[W], kp[W];
-    weights<T, W>(pc, W, beta, kt, kp);
+    weights64<W>(pc, beta, s_exp2, kt, kp);
     // joint footprint of the warp's points
     const int big = 1 << 30;
     const int rmin = __reduce_min_sync(0xffffffffu, act ? pc.r0 : big);
@@ -238,8 +280,8 @@ __global__ void __launch_bounds__(SPW_WARPS * 32)
     }
 }
 
-template <typename T, bool CPLX>
-static int launch_spread_warp(const cunusht_plan_s *P, int nreq, T *U, long long ubs, const double *loc, long long lbs,
+template <bool CPLX>
+static int launch_spread_warp(const cunusht_plan_s *P, int nreq, double *U, long long ubs, const double *loc, long long lbs,
                               long long npts, int layout, const double *gamma, int spin, const void *in,
                               long long ibs, int f32i, cudaStream_t st) {
     int lgn = 0;
@@ -247,17 +289,17 @@ static int launch_spread_warp(const cunusht_plan_s *P, int nreq, T *U, long long
     // strip: the footprint of 32 neighbouring ring pixels at about 2 fine
     // cells per pixel, plus row jitter from the deflection
     const int SR = P->w + 4, SC = 80 + P->w;
-    const size_t sm = (size_t)SPW_WARPS * SR * SC * (CPLX ? 2 : 1) * sizeof(T);
+    const size_t sm = (size_t)SPW_WARPS * SR * SC * (CPLX ? 2 : 1) * sizeof(double);
     const long long nwarps = (npts + 31) / 32;
     const unsigned nb = (unsigned)((nwarps + SPW_WARPS - 1) / SPW_WARPS);
     cudaError_t e = cudaSuccess;
     with_width(P->w, [&](auto WC) {
         constexpr int W = decltype(WC)::value;
-        if (sm > 48 * 1024)
-            e = cudaFuncSetAttribute(k_spread_warp<T, CPLX, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (sm + sizeof(float2) * 128 > 48 * 1024)  // with the static table
+            e = cudaFuncSetAttribute(k_spread_warp<CPLX, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e == cudaSuccess)
-            k_spread_warp<T, CPLX, W><<<dim3(nb, nreq), SPW_WARPS * 32, sm, st>>>(
-                U, P->nrows, P->Npf, P->Ntf, P->n_lo, W, (T)P->beta, loc, npts, layout, gamma, spin, in, f32i, SR, SC,
+            k_spread_warp<CPLX, W><<<dim3(nb, nreq), SPW_WARPS * 32, sm, st>>>(
+                U, P->nrows, P->Npf, P->Ntf, P->n_lo, P->beta, loc, npts, layout, gamma, spin, in, f32i, SR, SC,
                 ubs, lbs, ibs, P->spread_det ? P->d_ufix : nullptr, P->d_vmax, lgn);
     });
     CU_TRY(e);
@@ -639,12 +681,12 @@ int nufft_interp_batch(const cunusht_plan_s *P, int nreq, int spin, const void *
                                                                  out, f32o, ubs, lbs, obs);
         } else {
             if (spin == 0)
-                k_interp<double, false, W><<<grid, NU_TPB, 0, st>>>((const double *)U, P->nrows, P->Npf, P->Ntf,
-                                                                    P->n_lo, W, P->beta, loc, npts, layout, gamma,
+                k_interp<false, W><<<grid, NU_TPB, 0, st>>>((const double *)U, P->nrows, P->Npf, P->Ntf,
+                                                                    P->n_lo, P->beta, loc, npts, layout, gamma,
                                                                     spin, out, f32o, ubs, lbs, obs);
             else
-                k_interp<double, true, W><<<grid, NU_TPB, 0, st>>>((const double *)U, P->nrows, P->Npf, P->Ntf,
-                                                                   P->n_lo, W, P->beta, loc, npts, layout, gamma,
+                k_interp<true, W><<<grid, NU_TPB, 0, st>>>((const double *)U, P->nrows, P->Npf, P->Ntf,
+                                                                   P->n_lo, P->beta, loc, npts, layout, gamma,
                                                                    spin, out, f32o, ubs, lbs, obs);
         }
     });
@@ -679,8 +721,8 @@ int nufft_spread_batch(const cunusht_plan_s *P, int nreq, int spin, void *U, lon
         if (spin == 0) RC_TRY((launch_spread_warp_mixed<double, false>(P, nreq, (double *)U, ubs, loc, lbs, npts, layout, gamma, spin, in, ibs, f32i, st)));
         else RC_TRY((launch_spread_warp_mixed<double, true>(P, nreq, (double *)U, ubs, loc, lbs, npts, layout, gamma, spin, in, ibs, f32i, st)));
     } else {
-        if (spin == 0) RC_TRY((launch_spread_warp<double, false>(P, nreq, (double *)U, ubs, loc, lbs, npts, layout, gamma, spin, in, ibs, f32i, st)));
-        else RC_TRY((launch_spread_warp<double, true>(P, nreq, (double *)U, ubs, loc, lbs, npts, layout, gamma, spin, in, ibs, f32i, st)));
+        if (spin == 0) RC_TRY((launch_spread_warp<false>(P, nreq, (double *)U, ubs, loc, lbs, npts, layout, gamma, spin, in, ibs, f32i, st)));
+        else RC_TRY((launch_spread_warp<true>(P, nreq, (double *)U, ubs, loc, lbs, npts, layout, gamma, spin, in, ibs, f32i, st)));
     }
     CU_LAUNCH_CHECK();
     return spread_options_end(P, nreq, spin, U, ubs, npts, st);
@@ -696,8 +738,21 @@ int nufft_spread(const cunusht_plan_s *P, int spin, const double *loc, long long
 // pixel instead of one per ring); the rotation angle gamma of
 // CPU_nufft_transformer.py:160 is computed as a single atan2 of the angle
 // difference (equal modulo 2 pi).
+// geo (may be NULL): per ring sin, cos, cot of the colatitude and the pixel spacing, from the plan.
+// FP64 instructions bound it: about 330 per pixel with sincos, three atan2 and the divisions by
+// constants, about 100 with ring tables and series of the increments; 8.4 M pixels 4.46 -> 1.31 ms.
+__device__ __forceinline__ double asin_small(double x) {  // |x| < 0.02: error below 1e-20
+    const double x2 = x * x;
+    return x + x * x2 * (1.0 / 6.0 + x2 * (3.0 / 40.0 + x2 * (15.0 / 336.0 + x2 * (105.0 / 3456.0))));
+}
+__device__ __forceinline__ double atan_small(double x) {
+    const double x2 = x * x;
+    return x + x * x2 * (-1.0 / 3.0 + x2 * (1.0 / 5.0 + x2 * (-1.0 / 7.0 + x2 * (1.0 / 9.0))));
+}
+
 __global__ void __launch_bounds__(256)
-    k_pointing(int nring, const double *__restrict__ rth, const double *__restrict__ rph0,
+    k_pointing(int nring, int nph_uniform, const RingGeo *__restrict__ geo, const double *__restrict__ rth,
+               const double *__restrict__ rph0,
                const long long *__restrict__ rnph, const long long *__restrict__ rofs, long long npix,
                const double *__restrict__ dth, const double *__restrict__ dph,
                double *__restrict__ oth, double *__restrict__ oph, double *__restrict__ ogam, long long dbs,
@@ -709,43 +764,63 @@ __global__ void __launch_bounds__(256)
     oth += blockIdx.y * pbs;
     oph += blockIdx.y * pbs;
     if (ogam) ogam += blockIdx.y * npix;
-    int lo = 0, hi = nring - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (rofs[mid] <= j) lo = mid;
-        else hi = mid - 1;
+    int ring;
+    if (nph_uniform > 0) {
+        ring = j < 0x7FFFFFFFLL ? (int)((unsigned)j / (unsigned)nph_uniform) : (int)(j / nph_uniform);
+    } else {
+        int lo = 0, hi = nring - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (rofs[mid] <= j) lo = mid;
+            else hi = mid - 1;
+        }
+        ring = lo;
     }
-    const int ring = lo;
     const double theta = rth[ring];
-    const long long nph = rnph[ring];
-    const double phi = rph0[ring] + (double)(j - rofs[ring]) * (TWOPI / (double)nph);
+    double st, ct, cot, dphi;
+    if (geo) {
+        const RingGeo g = geo[ring];
+        st = g.st, ct = g.ct, cot = g.cot, dphi = g.dphi;
+    } else {
+        sincos(theta, &st, &ct);
+        cot = ct / st;
+        dphi = TWOPI / (double)rnph[ring];
+    }
+    const double phi = rph0[ring] + (double)(j - rofs[ring]) * dphi;
     const double t = dth[j], p = dph[j];
     const double d2 = t * t + p * p;
-    double sinaoa, cosa;
-    if (d2 > 1e-6) {
-        const double a = sqrt(d2);
-        double sa;
-        sincos(a, &sa, &cosa);
-        sinaoa = sa / a;
+    double sinaoa, cm1;  // sin(a) / a, cos(a) - 1
+    if (d2 < 1e-2) {
+        // series, error below d2^5 / 10! < 3e-17
+        sinaoa = 1.0 + d2 * (-1.0 / 6.0 + d2 * (1.0 / 120.0 + d2 * (-1.0 / 5040.0 + d2 * (1.0 / 362880.0))));
+        cm1 = d2 * (-0.5 + d2 * (1.0 / 24.0 + d2 * (-1.0 / 720.0 + d2 * (1.0 / 40320.0))));
     } else {
-        // sin(a)/a and cos(a) series, error < a^10/10!
-        sinaoa = 1.0 - d2 / 6.0 * (1.0 - d2 / 20.0 * (1.0 - d2 / 42.0 * (1.0 - d2 / 72.0)));
-        cosa = 1.0 - d2 / 2.0 * (1.0 - d2 / 12.0 * (1.0 - d2 / 30.0 * (1.0 - d2 / 56.0)));
+        const double a = sqrt(d2);
+        double sa, ca;
+        sincos(a, &sa, &ca);
+        sinaoa = sa / a;
+        cm1 = ca - 1.0;
     }
-    double st, ct;
-    sincos(theta, &st, &ct);
+    const double cosa = 1.0 + cm1;
     const double nx = st * cosa + ct * t * sinaoa;
     const double ny = -p * sinaoa;
     const double nz = ct * cosa - st * t * sinaoa;
-    oth[j] = atan2(sqrt(nx * nx + ny * ny), nz);
-    double php = phi - atan2(ny, nx);
+    const double rho = sqrt(nx * nx + ny * ny);
+    // the increments from their series where they are small (all but the pixels next to a pole):
+    // theta' - theta = asin(rho ct - nz st), phi' - phi = -atan(ny / nx)
+    const double sd = rho * ct - nz * st;
+    oth[j] = fabs(sd) < 0.02 ? theta + asin_small(sd) : atan2(rho, nz);
+    const double q = ny / nx;
+    double php = phi - (nx > 0.0 && fabs(q) < 0.02 ? atan_small(q) : atan2(ny, nx));
     if (php >= TWOPI) php -= TWOPI;
     oph[j] = php;
     if (ogam) {
         // gamma = atan2(p, t) - atan2(p, d sin d cot(theta) + t cos d)
-        //       = atan2(p * x2 - t * p, t * x2 + p * p),  x2 = d^2 (sin d / d) cot + t cos d
-        const double x2 = d2 * sinaoa * (ct / st) + t * cosa;
-        ogam[j] = (d2 > 0.0) ? atan2(p * x2 - t * p, t * x2 + p * p) : 0.0;
+        //       = atan2(p (x2 - t), t * x2 + p * p),  x2 - t = d^2 (sin d / d) cot + t (cos d - 1)
+        const double x2m = d2 * sinaoa * cot + t * cm1;
+        const double num = p * x2m, den = t * (t + x2m) + p * p;
+        const double g = num / den;
+        ogam[j] = d2 > 0.0 ? (den > 0.0 && fabs(g) < 0.02 ? atan_small(g) : atan2(num, den)) : 0.0;
     }
 }
 
@@ -878,6 +953,7 @@ __global__ void __launch_bounds__(256)
 // derivatives f_theta, f_phi of the unlensed field at the deflected points
 // are interpolated from the same fine grid with the derivative of the same
 // ES kernel, so this is the exact derivative of the implemented forward map.
+// Kernel values and derivatives as in weights64, the width a run-time value.
 template <typename TU>
 __global__ void __launch_bounds__(256)
     k_lens_vjp_s0(const TU *__restrict__ U, int nrows, int Npf, int Ntf, int n_lo, int w, double beta,
@@ -885,6 +961,9 @@ __global__ void __launch_bounds__(256)
                   const long long *__restrict__ rnph, const long long *__restrict__ rofs, long long npix,
                   const double *__restrict__ dth, const double *__restrict__ dph,
                   const double *__restrict__ ptg, const double *__restrict__ grad, double *__restrict__ gd) {
+    __shared__ float2 s_exp2[128];
+    if (threadIdx.x < 128) s_exp2[threadIdx.x] = ES_EXP2[threadIdx.x];
+    __syncthreads();
     const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= npix) return;
     int lo = 0, hi = nring - 1;
@@ -901,9 +980,21 @@ __global__ void __launch_bounds__(256)
     double kt[MAXW], dkt[MAXW], kp[MAXW], dkp[MAXW];
     const double sc = 2.0 / w;
     const double dzt = -sc * Ntf / TWOPI, dzp = -sc * Npf / TWOPI;  // dz / dtheta, dz / dphi
-#pragma unroll
-    for (int a = 0; a < MAXW; ++a) {
-        if (a < w) {
+    if (w <= ES_SPLIT_MAXW) {
+        const EsParams E{df_from(sc), df_from(-beta)};
+        const dfl f0 = df_from(pc.ft), f1 = df_from(pc.fp);
+#pragma unroll 1
+        for (int a = 0; a < w; ++a) {
+            dfl g, v = es_kernel_df<true>(f0, (float)a, E, s_exp2, &g);
+            kt[a] = df_to(v);
+            dkt[a] = df_to(df_mul(v, g)) * dzt;
+            v = es_kernel_df<true>(f1, (float)a, E, s_exp2, &g);
+            kp[a] = df_to(v);
+            dkp[a] = df_to(df_mul(v, g)) * dzp;
+        }
+    } else {
+#pragma unroll 1
+        for (int a = 0; a < w; ++a) {
             const double zt = (pc.ft + a) * sc, zp = (pc.fp + a) * sc;
             const double qt = 1.0 - zt * zt, qp = 1.0 - zp * zp;
             const double rt = qt > 0.0 ? sqrt(qt) : 0.0, rp = qp > 0.0 ? sqrt(qp) : 0.0;
@@ -917,15 +1008,12 @@ __global__ void __launch_bounds__(256)
     for (int a = 0; a < w; ++a) {
         const TU *row = U + (long long)(pc.r0 + a) * Npf;
         double r0 = 0.0, r1 = 0.0;
-#pragma unroll
-        for (int b = 0; b < MAXW; ++b) {
-            if (b < w) {
-                int c = pc.p0 + b;
-                c = c < 0 ? c + Npf : (c >= Npf ? c - Npf : c);
-                const double v = (double)row[c];
-                r0 = fma(kp[b], v, r0);
-                r1 = fma(dkp[b], v, r1);
-            }
+        for (int b = 0; b < w; ++b) {
+            int c = pc.p0 + b;
+            c = c < 0 ? c + Npf : (c >= Npf ? c - Npf : c);
+            const double v = (double)row[c];
+            r0 = fma(kp[b], v, r0);
+            r1 = fma(dkp[b], v, r1);
         }
         ft = fma(dkt[a], r0, ft);
         fp = fma(kt[a], r1, fp);
@@ -975,16 +1063,13 @@ __global__ void __launch_bounds__(256)
 
 int lens_vjp_launch(const cunusht_plan_s *P, const double *ptg, const double *grad, double *gd, cudaStream_t st) {
     const int nb = (int)((P->npix + 255) / 256);
-    if (P->fwd_u32 || P->grid_fp32)
-        k_lens_vjp_s0<float><<<nb, 256, 0, st>>>((const float *)P->d_U, P->nrows, P->Npf, P->Ntf, P->n_lo, P->w,
-                                                 P->beta, P->nring, P->d_ring_theta, P->d_ring_phi0, P->d_ring_nph,
-                                                 P->d_ring_ofs, P->npix, P->d_glmap, P->d_glmap + P->npix, ptg, grad,
-                                                 gd);
-    else
-        k_lens_vjp_s0<double><<<nb, 256, 0, st>>>((const double *)P->d_U, P->nrows, P->Npf, P->Ntf, P->n_lo, P->w,
-                                                  P->beta, P->nring, P->d_ring_theta, P->d_ring_phi0, P->d_ring_nph,
-                                                  P->d_ring_ofs, P->npix, P->d_glmap, P->d_glmap + P->npix, ptg,
-                                                  grad, gd);
+    auto launch = [&](auto kern, const auto *U) {
+        kern<<<nb, 256, 0, st>>>(U, P->nrows, P->Npf, P->Ntf, P->n_lo, P->w, P->beta, P->nring, P->d_ring_theta,
+                                 P->d_ring_phi0, P->d_ring_nph, P->d_ring_ofs, P->npix, P->d_glmap,
+                                 P->d_glmap + P->npix, ptg, grad, gd);
+    };
+    if (P->fwd_u32 || P->grid_fp32) launch(k_lens_vjp_s0<float>, (const float *)P->d_U);
+    else launch(k_lens_vjp_s0<double>, (const double *)P->d_U);
     CU_LAUNCH_CHECK();
     return CUNUSHT_OK;
 }
@@ -998,8 +1083,9 @@ int pointing_batch(const cunusht_plan_s *P, int nreq, const double *d, long long
                                                P->d_ring_nph, P->d_ring_ofs, P->npix, d, d + P->npix, ptg,
                                                ptg + P->npix, gamma, dbs, pbs);
     else
-        k_pointing<<<grid, 256, 0, st>>>(P->nring, P->d_ring_theta, P->d_ring_phi0, P->d_ring_nph, P->d_ring_ofs,
-                                         P->npix, d, d + P->npix, ptg, ptg + P->npix, gamma, dbs, pbs);
+        k_pointing<<<grid, 256, 0, st>>>(P->nring, P->nph_uniform, P->d_ring_geo, P->d_ring_theta, P->d_ring_phi0,
+                                         P->d_ring_nph, P->d_ring_ofs, P->npix, d, d + P->npix, ptg, ptg + P->npix,
+                                         gamma, dbs, pbs);
     CU_LAUNCH_CHECK();
     return CUNUSHT_OK;
 }
@@ -1015,12 +1101,13 @@ int pointing_mixed_launch(int nring, int nph_uniform, const double *rth, const f
     return CUNUSHT_OK;
 }
 
-int pointing_launch(int nring, const double *rth, const double *rph0, const long long *rnph,
-                    const long long *rofs, long long npix, const double *dth, const double *dph,
+int pointing_launch(int nring, int nph_uniform, const RingGeo *geo, const double *rth, const double *rph0,
+                    const long long *rnph, const long long *rofs, long long npix, const double *dth, const double *dph,
                     double *out_th, double *out_ph, double *out_gamma, cudaStream_t st) {
     if (npix == 0) return CUNUSHT_OK;
     const int nb = (int)((npix + 255) / 256);
-    k_pointing<<<nb, 256, 0, st>>>(nring, rth, rph0, rnph, rofs, npix, dth, dph, out_th, out_ph, out_gamma, 0, 0);
+    k_pointing<<<nb, 256, 0, st>>>(nring, nph_uniform, geo, rth, rph0, rnph, rofs, npix, dth, dph, out_th, out_ph,
+                                   out_gamma, 0, 0);
     CU_LAUNCH_CHECK();
     return CUNUSHT_OK;
 }

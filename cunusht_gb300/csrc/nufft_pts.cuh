@@ -31,7 +31,7 @@ __device__ __forceinline__ PointCoords point_coords(double th, double ph, int Nt
     double t = th * ((double)Ntf / TWOPI);
     t = fmin(fmax(t, -1.0), 0.5 * Ntf + 1.0);
     double p = ph * ((double)Npf / TWOPI);
-    p -= floor(p / (double)Npf) * (double)Npf;
+    p -= floor(p * (1.0 / (double)Npf)) * (double)Npf;  // Npf a power of two: exact
     p = fmin(fmax(p, 0.0), (double)Npf);
     const double hw = 0.5 * w;
     const int n0 = (int)ceil(t - hw);
@@ -116,6 +116,104 @@ __device__ __forceinline__ float es_kernel_acc(float z, float beta) {
     if (q <= 0.f) return 0.f;
     const float r = sqrtf(q);
     return expf(-beta * (z * z) / (1.f + r));
+}
+
+// 2^(j / 128) as double-floats
+__device__ const float2 ES_EXP2[128] = {
+    {0x1.0p+0f, 0x0.0p+0f}, {0x1.0163dap+0f, 0x1.3f6666p-25f}, {0x1.02c9a4p+0f, -0x1.887fap-28f},
+    {0x1.04315ep+0f, 0x1.0dcffp-25f}, {0x1.059b0ep+0f, -0x1.9d4f52p-25f}, {0x1.0706b2p+0f, 0x1.3bbedcp-25f},
+    {0x1.087452p+0f, -0x1.e2990ep-26f}, {0x1.09e3ecp+0f, 0x1.58de7p-25f}, {0x1.0b5586p+0f, 0x1.9f3122p-25f},
+    {0x1.0cc922p+0f, 0x1.6e48fep-25f}, {0x1.0e3ec4p+0f, -0x1.a585ccp-25f}, {0x1.0fb66ap+0f, 0x1.ffda64p-25f},
+    {0x1.11301ep+0f, -0x1.fdb496p-25f}, {0x1.12abdcp+0f, 0x1.b0c73p-30f}, {0x1.1429aap+0f, 0x1.d525bcp-25f},
+    {0x1.15a98cp+0f, 0x1.14b1cap-25f}, {0x1.172b84p+0f, -0x1.c15742p-27f}, {0x1.18af94p+0f, -0x1.dcdc86p-26f},
+    {0x1.1a35bep+0f, 0x1.6df96ep-25f}, {0x1.1bbe08p+0f, 0x1.011734p-26f}, {0x1.1d4874p+0f, -0x1.d2e8cap-25f},
+    {0x1.1ed502p+0f, 0x1.7e6c8ep-27f}, {0x1.2063b8p+0f, 0x1.0c519ap-25f}, {0x1.21f49ap+0f, -0x1.d0446ep-25f},
+    {0x1.2387a6p+0f, 0x1.ceac48p-25f}, {0x1.251ce4p+0f, 0x1.f654c8p-25f}, {0x1.26b456p+0f, 0x1.789f38p-26f},
+    {0x1.284dfep+0f, 0x1.f5638p-28f}, {0x1.29e9ep+0f, -0x1.5c0424p-25f}, {0x1.2b87fep+0f, -0x1.e4a4cep-25f},
+    {0x1.2d285ap+0f, 0x1.b900c2p-26f}, {0x1.2ecafap+0f, 0x1.27c5eap-25f}, {0x1.306fep+0f, 0x1.4636e2p-25f},
+    {0x1.32171p+0f, -0x1.d993e8p-27f}, {0x1.33c08cp+0f, -0x1.b37d2p-25f}, {0x1.356c56p+0f, -0x1.b5803cp-30f},
+    {0x1.371a74p+0f, -0x1.18aac6p-25f}, {0x1.38cae6p+0f, 0x1.a0bb0cp-25f}, {0x1.3a7db4p+0f, -0x1.634c02p-25f},
+    {0x1.3c32dcp+0f, 0x1.89d472p-27f}, {0x1.3dea64p+0f, 0x1.824684p-25f}, {0x1.3fa45p+0f, 0x1.2b2006p-26f},
+    {0x1.4160a2p+0f, 0x1.f72e2ap-28f}, {0x1.431f5ep+0f, -0x1.abd5dap-26f}, {0x1.44e086p+0f, 0x1.8624b4p-30f},
+    {0x1.46a41ep+0f, 0x1.a3a00ap-25f}, {0x1.486a2cp+0f, -0x1.47d866p-25f}, {0x1.4a32bp+0f, -0x1.e50584p-25f},
+    {0x1.4bfdaep+0f, -0x1.593abcp-25f}, {0x1.4dcb2ap+0f, -0x1.8088bcp-26f}, {0x1.4f9b28p+0f, -0x1.2c5a6cp-25f},
+    {0x1.516daap+0f, 0x1.67b32p-27f}, {0x1.5342b6p+0f, -0x1.2c561p-25f}, {0x1.551a4cp+0f, 0x1.4bb242p-25f},
+    {0x1.56f474p+0f, -0x1.295b04p-25f}, {0x1.58d12ep+0f, -0x1.6d07p-25f}, {0x1.5ab07ep+0f, -0x1.5bd5ecp-27f},
+    {0x1.5c9268p+0f, 0x1.4b28d6p-25f}, {0x1.5e76f2p+0f, -0x1.4a5bd6p-25f}, {0x1.605e1cp+0f, -0x1.a248fep-26f},
+    {0x1.6247ecp+0f, -0x1.f8b55p-25f}, {0x1.643464p+0f, -0x1.66679cp-25f}, {0x1.662388p+0f, 0x1.2a9112p-27f},
+    {0x1.68155ep+0f, -0x1.766ad2p-25f}, {0x1.6a09e6p+0f, 0x1.9fcef4p-26f}, {0x1.6c0128p+0f, -0x1.5e84a8p-25f},
+    {0x1.6dfb24p+0f, -0x1.cd72e8p-27f}, {0x1.6ff7ep+0f, -0x1.ab9aep-26f}, {0x1.71f75ep+0f, 0x1.1d8beep-25f},
+    {0x1.73f9a4p+0f, 0x1.14b02ep-25f}, {0x1.75feb6p+0f, -0x1.37b306p-25f}, {0x1.780694p+0f, 0x1.fbcba8p-25f},
+    {0x1.7a1148p+0f, -0x1.829fdp-25f}, {0x1.7c1edp+0f, 0x1.30c132p-28f}, {0x1.7e2f34p+0f, -0x1.261634p-25f},
+    {0x1.804276p+0f, -0x1.783cbep-25f}, {0x1.82589ap+0f, -0x1.accc7cp-26f}, {0x1.8471a4p+0f, 0x1.88f1ecp-26f},
+    {0x1.868d9ap+0f, -0x1.2edb44p-26f}, {0x1.88ac7ep+0f, -0x1.9d665ap-26f}, {0x1.8ace54p+0f, 0x1.15506ep-27f},
+    {0x1.8cf322p+0f, -0x1.29576ep-25f}, {0x1.8f1aeap+0f, -0x1.baa232p-26f}, {0x1.9145bp+0f, 0x1.723ff8p-25f},
+    {0x1.93737cp+0f, -0x1.e64744p-25f}, {0x1.95a44cp+0f, 0x1.790a42p-25f}, {0x1.97d82ap+0f, -0x1.0d8d84p-31f},
+    {0x1.9a0f18p+0f, -0x1.e6bf08p-25f}, {0x1.9c4918p+0f, 0x1.51f848p-27f}, {0x1.9e8632p+0f, -0x1.873738p-26f},
+    {0x1.a0c668p+0f, -0x1.2886a6p-26f}, {0x1.a309bep+0f, 0x1.8945a6p-25f}, {0x1.a5503cp+0f, -0x1.b83b54p-25f},
+    {0x1.a799e2p+0f, -0x1.99e994p-25f}, {0x1.a9e6b6p+0f, -0x1.50c048p-25f}, {0x1.ac36bcp+0f, -0x1.606432p-31f},
+    {0x1.ae89fap+0f, -0x1.a94b14p-26f}, {0x1.b0e072p+0f, 0x1.31b6ccp-25f}, {0x1.b33a2cp+0f, -0x1.ec3a82p-26f},
+    {0x1.b59728p+0f, 0x1.bcab28p-25f}, {0x1.b7f77p+0f, -0x1.a09438p-25f}, {0x1.ba5b04p+0f, -0x1.ebdf36p-25f},
+    {0x1.bcc1eap+0f, -0x1.f687c6p-25f}, {0x1.bf2c26p+0f, -0x1.0a387ep-26f}, {0x1.c199bep+0f, -0x1.3d56b2p-27f},
+    {0x1.c40ab6p+0f, -0x1.7c2c98p-39f}, {0x1.c67f12p+0f, 0x1.cafa2ap-25f}, {0x1.c8f6dap+0f, -0x1.7f230ap-25f},
+    {0x1.cb720ep+0f, -0x1.8837ccp-27f}, {0x1.cdf0b6p+0f, -0x1.54478p-25f}, {0x1.d072d4p+0f, 0x1.40f13p-25f},
+    {0x1.d2f87p+0f, 0x1.01b13ep-25f}, {0x1.d5818ep+0f, -0x1.822dbcp-27f}, {0x1.d80e32p+0f, -0x1.26cf8ep-25f},
+    {0x1.da9e6p+0f, 0x1.ed9942p-27f}, {0x1.dd322p+0f, -0x1.9fc974p-25f}, {0x1.dfc974p+0f, -0x1.908c94p-25f},
+    {0x1.e26462p+0f, -0x1.614bdap-25f}, {0x1.e502eep+0f, 0x1.e2cffep-26f}, {0x1.e7a52p+0f, -0x1.0e2cep-26f},
+    {0x1.ea4afap+0f, 0x1.52486cp-27f}, {0x1.ecf482p+0f, 0x1.b1ccfep-25f}, {0x1.efa1bep+0f, 0x1.cc2b44p-25f},
+    {0x1.f252b4p+0f, -0x1.1288aep-25f}, {0x1.f50766p+0f, -0x1.246ebp-26f}, {0x1.f7bfdap+0f, 0x1.b397c2p-25f},
+    {0x1.fa7c18p+0f, 0x1.9e90d8p-28f}, {0x1.fd3c22p+0f, 0x1.71ee3ep-25f}};
+
+// The kernel value of the FP64 plans from double-float arithmetic on the FP32
+// pipe: about 100 FP32 instructions for the value (absolute error 2e-14, of
+// values up to 1) in place of about 33 FP64 instructions of exp, sqrt and
+// products, each of which takes the issue time of 64 (2 FP64 lanes per SM and
+// clock, measured).  z = (a + f) s with f the offset of the first tap and s =
+// 2 / w; exponent y = -beta z^2 / (1 + sqrt(1 - z^2)) (no cancellation); e^y =
+// 2^k (2^(j/128)) e^f from the table T in shared memory with |f| < 0.0028, ln 2
+// / 128 split so that the first two products are exact.  Used for widths up to
+// ES_SPLIT_MAXW (eps >= 1e-10), where the kernel's own aliasing error is over a
+// hundred times larger; wider kernels keep the FP64 functions.
+constexpr int ES_SPLIT_MAXW = 12;
+struct EsParams {
+    dfl s, nbeta;  // 2 / w, -beta
+};
+template <bool DERIV>
+__device__ __forceinline__ dfl es_kernel_df(dfl f0, float a, const EsParams &E, const float2 *T, dfl *dlog) {
+    const dfl z = df_mul(df_add(dfl{a, 0.f}, f0), E.s);
+    const dfl z2 = df_mul(z, z);
+    dfl q = df_fast(1.f, -z2.h);
+    q = df_fast(q.h, q.l - z2.l);
+    if (DERIV) *dlog = dfl{0.f, 0.f};
+    if (!(q.h > 0.f)) return dfl{0.f, 0.f};
+    const float r0 = sqrtf(q.h);
+    const dfl r = df_fast(r0, (fmaf(-r0, r0, q.h) + q.l) / (2.f * r0));
+    dfl d = df_fast(1.f, r.h);
+    d.l += r.l;
+    const dfl bz = df_mul(E.nbeta, z2);
+    const float i0 = 1.f / d.h;
+    const float y0 = bz.h * i0;
+    const dfl y = df_fast(y0, (fmaf(-y0, d.l, fmaf(-y0, d.h, bz.h)) + bz.l) * i0);
+    if (DERIV) {  // d log(psi) / dz = -beta z / sqrt(1 - z^2)
+        const dfl n = df_mul(E.nbeta, z);
+        const float g0 = n.h / r.h;
+        *dlog = df_fast(g0, (fmaf(-g0, r.l, fmaf(-g0, r.h, n.h)) + n.l) / r.h);
+    }
+    const float k = rintf(y.h * 184.664965f);  // 128 / ln 2
+    const float f1 = fmaf(-k, 0x1.62cp-8f, y.h);
+    const dfl f2 = df_add_u(dfl{f1, y.l}, dfl{-(k * 0x1.214p-19f), -(k * 0x1.fbe8e8p-30f)});
+    const dfl f = df_fast(f2.h, f2.l);
+    const float qq = f.h * f.h;
+    const float qe = fmaf(f.h, f.l + f.l, fmaf(f.h, f.h, -qq));
+    const float c3 = f.h * qq * (1.f / 6.f);
+    const float small = fmaf(0.5f, qe, fmaf(c3, 0.25f * f.h, c3)) + f.l;
+    const dfl p = df_fast(f.h, 0.5f * qq);  // e^f - 1 = p.h + (p.l + small)
+    const int ki = (int)k;
+    const float2 t = T[ki & 127];
+    const dfl tp = df_mul_u(dfl{t.x, t.y}, dfl{p.h, p.l + small});
+    dfl v = df_fast(t.x, tp.h);
+    v.l += tp.l + t.y;
+    return df_scale(v, __int_as_float((127 + (ki >> 7)) << 23));  // k / 128 >= -54
 }
 
 // Fixed-point accumulation of the deterministic spreading: every cell sum is
