@@ -166,6 +166,62 @@ __device__ __forceinline__ void fft_pass_e(cplx<T> *buf, int N, int Ns, int dir,
     __syncthreads();
 }
 
+// One radix-16 pass of the FP64 and double-float transforms with 16 elements
+// per thread: two radix-4 stages in registers, so it costs the shared-memory
+// round trip and the two barriers of one pass for the work of two.  Element
+// r = 4 a + b of the butterfly: radix-4 over a with the twiddles w^(4 a k), the
+// factors e^{dir 2 pi i b q / 16} w^(b k), radix-4 over b.  In place in v, whose
+// slot 4 q + p then holds output q + 4 p.
+template <typename T>
+__device__ __forceinline__ void fft_pass16(cplx<T> *buf, int N, int Ns, int dir, const cplx<T> *__restrict__ stw, int M,
+                                           int nthr) {
+    using C = cplx<T>;
+    const int nb = N / 16;  // == nthr
+    const bool act = (int)threadIdx.x < nthr;
+    const int j = threadIdx.x;
+    C v[16];
+    if (act) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) v[(r & 3) * 4 + (r >> 2)] = buf[j + r * nb];  // slot 4 b + a
+    }
+    __syncthreads();
+    if (act) {
+        const int tstep = M / (Ns * 16);
+        const int lq = __ffs(M) - 3;  // log2(M / 4)
+        const int k = j & (Ns - 1), t1 = k * tstep;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            C *u = v + 4 * b;
+            if (Ns > 1) {
+#pragma unroll
+                for (int a = 1; a < 4; ++a) {
+                    C w = tw_quarter<T>(stw, 4 * a * t1, lq);
+                    if (dir > 0) w.y = -w.y;
+                    u[a] = cmul(u[a], w);
+                }
+            }
+            dft4(u[0], u[1], u[2], u[3], dir);  // u[q]: frequency q over a
+            asm volatile("" ::: "memory");
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+#pragma unroll
+            for (int b = 1; b < 4; ++b) {
+                // w^(b k) e^{-2 pi i b q / 16}: table index b (t1 + q M / 16)
+                C w = tw_quarter<T>(stw, b * (t1 + q * (M >> 4)), lq);
+                if (dir > 0) w.y = -w.y;
+                v[4 * b + q] = cmul(v[4 * b + q], w);
+            }
+            dft4(v[q], v[4 + q], v[8 + q], v[12 + q], dir);
+            const int idxD = (j - k) * 16 + k;
+#pragma unroll
+            for (int p = 0; p < 4; ++p) buf[idxD + (q + 4 * p) * Ns] = v[4 * p + q];
+            asm volatile("" ::: "memory");
+        }
+    }
+    __syncthreads();
+}
+
 // Whole transform with E elements per thread; radices up to min(E, RMAX) with
 // RMAX = 16 for float and 8 for double / double-float (register budget).
 // l0 > 0: the first passes, of 2^l0 points in all, are already done (buf
@@ -178,6 +234,13 @@ __device__ __forceinline__ void fft_smem_e(cplx<T> *buf, int N, int dir, const c
     const int nthr = N / E;
     int rem = __ffs(N) - 1 - l0;
     int Ns = 1 << l0;
+    if constexpr (E == 16 && !std::is_same<T, float>::value) {
+        while (rem >= 4) {
+            fft_pass16<T>(buf, N, Ns, dir, stw, M, nthr);
+            Ns <<= 4;
+            rem -= 4;
+        }
+    }
     while (rem > 0) {
         const int r = rem < LR ? rem : LR;
         if (r == 4) {
