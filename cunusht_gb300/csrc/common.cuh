@@ -151,6 +151,10 @@ constexpr int MR_NMAX = 8192;
 constexpr int MR_MAXST = 16;
 constexpr int MR_KMAX = 128;
 
+namespace cunusht {
+struct FixCoef;  // rec64.cuh
+}
+
 // sin, cos and cot of a ring's colatitude, pixel spacing 2 pi / nph
 struct RingGeo {
     double st, ct, cot, dphi;
@@ -234,7 +238,9 @@ struct cunusht_plan_s {
     int *d_t6_woff[3] = {};
     double2 *d_t6_ag[3] = {};
     double *d_t6_cl[3] = {};
+    cunusht::FixCoef *d_t6_fx[3] = {};  // (a_l, g_l) in fixed point
     short *d_t6_eb[3] = {};     // digit exponent of mu per (m, chunk of 16 l)
+    short *d_t6_es[3] = {};     // the largest of each m
     double2 *d_t6_lg0[3] = {};  // per m: log2 start normalisation (hi, lo)
     RingLog *d_t6_lsc[2] = {};  // per [grid][pair]: log2 sin(theta/2), log2 cos(theta/2), (hi, lo) each
     std::vector<double> h_gl_theta, h_cc_theta;  // theta of the ring pairs

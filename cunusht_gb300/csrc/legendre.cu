@@ -1098,6 +1098,15 @@ int leg_synth_spin_df_pairs(const cunusht_plan_s *P, int nb, int npairs, const d
     return CUNUSHT_OK;
 }
 
+// FP64 plans go to the tensor cores unless the work is a few microseconds:
+// below lmax 56 a spin-0 transform is quicker in the one launch of the
+// CUDA-core kernel than in records, pole pair and main kernel (synthesis lmax
+// 31: 31 against 35 us, 47: 33 against 37, 63: 39 against 37; spin 2 at 31: 43
+// against 36).
+static bool f64_tensor_cores(const cunusht_plan_s *P, int spin) {
+    return P->use_tc && P->d_t6_ag[spin] && (spin > 0 || P->lmax >= 56);
+}
+
 // nreq requests (alm at G + r * astride, columns at H + r * hstride); the
 // mixed-precision kernels process several requests per launch with one shared
 // recursion (tensor cores: up to eight, CUDA cores: up to four), the FP64
@@ -1150,7 +1159,7 @@ int leg_synth_batch_fl(const cunusht_plan_s *P, int nreq, int spin, const double
     for (int r = 0; r < nreq; ++r) {
         const double2 *Gr = G + r * astride, *Cr = C ? C + r * astride : nullptr;
         double2 *Hr = H + r * hstride;
-        if (P->use_tc && P->d_t6_ag[spin])
+        if (f64_tensor_cores(P, spin))
             RC_TRY(leg_synth_tc64(P, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.ld, R.pole, R.pole_rn, R.pole_rs, cc,
                                   spin, Gr, Cr, lf, Hr, st));
         else
@@ -1312,7 +1321,7 @@ int leg_adjoint_batch(const cunusht_plan_s *P, int nreq, int spin, int ncomp, co
     for (int r = 0; r < nreq; ++r) {
         const double2 *Hr = H + r * hstride;
         double2 *Gr = G + r * astride, *Cr = (spin > 0 && ncomp > 1) ? C + r * astride : nullptr;
-        if (P->use_tc && P->d_t6_ag[spin])
+        if (f64_tensor_cores(P, spin))
             RC_TRY(leg_adjoint_tc64(P, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.ld, R.pole, R.pole_rn, R.pole_rs, cc,
                                     spin, ncomp, Hr, lf, Gr, Cr, st));
         else

@@ -5,10 +5,14 @@
 //
 // GB300 issues FP64 at 2 lanes per SM and clock, so the FP64 pipe bounds the
 // CUDA-core kernel (legendre.cu): 14 FP64 instructions per (l, m, ring pair)
-// for spin s, 8 of them the contraction and 6 the two recursions.  Here
+// for spin s, 8 of them the contraction and 6 the two recursions (88.7 ms at
+// lmax 2047 spin 2).  Here
 //   * the recursion is rescaled, lambda_l = c_l mu_l with c_{l+1} = beta_l
 //     c_{l-1}, to mu_{l+1} = (a_l x + g_l) mu_l - mu_{l-1}: 2 FP64
-//     instructions per step and ring instead of 3 (c_l goes into the alm);
+//     instructions per step and ring instead of 3 (c_l goes into the alm), and
+//     past the turning point it runs in 64-bit fixed point without any
+//     (rec64.cuh: 22.8 against 37.1 clocks per step of a warp and SM, digits
+//     included); a warp goes over when all its rings have;
 //   * mu and the alm are split into seven 8-bit digits on the integer pipe
 //     (rec64.cuh) and multiplied on the tensor cores,
 //         mu = 2^El 2^-7 sum_i d_i 2^-8i,   c a = 2^Ea 2^-7 sum_j t_j 2^-8j,
@@ -22,9 +26,13 @@
 // The products carry 2^-56 of the bounds and the sum over l rounds twice per
 // 128 terms instead of once per term.
 //
-// Layout as in legendre_tc.cu: one order m and 512 rings per block as four
-// 128-row MMA tiles, one ring per thread (spin s: 256 pairs, both rings; spin
-// 0: 512 pairs, the theta ring only), chunks of 8 l: A rows hold eight 16-byte
+// lmax 2047 spin 2, one request: 9.7 ms (FP64 recursion throughout, one block
+// of 512 rings per SM: 13.2 ms; two of 256: 12.3 ms; fixed point in half of the
+// warps, to share the work between the FP64 and integer pipes: 9.9 ms).
+//
+// Layout as in legendre_tc.cu: one order m and 256 rings per block as two
+// 128-row MMA tiles, two blocks per SM, one ring per thread (spin s: 128 pairs,
+// both rings; spin 0: 256 pairs, the theta ring only), chunks of 8 l: A rows hold eight 16-byte
 // K-cores (digit i, 8 l), the eighth zero, so a chunk is four MMA K-steps; B'
 // rows (weight g, column) hold t_{g-i} at K-core i.  Two A / B' buffers with
 // full (one arrival per ring warp) and empty (commit) mbarriers; the window
@@ -50,7 +58,7 @@ constexpr int T6_CPW = T6_W / T6_KC;      // chunks per window
 constexpr int T6_ND = 7;                  // digits, and digit-product weights kept
 constexpr int T6_NO = 4;                  // outputs per ring
 constexpr int T6_NN = 32;                 // MMA N: 7 x 4 weights x outputs, padded
-constexpr int T6_NT = 4;                  // 128-ring tiles per block
+constexpr int T6_NT = 2;                  // 128-ring tiles per block
 constexpr int T6_T = 128 * T6_NT;         // ring threads
 constexpr int T6_BLOCK = T6_T + 32;       // + the MMA warp
 constexpr int T6_TILE = 128 * 128;        // A tile: 128 rows x 8 K-cores x 16 bytes
@@ -59,11 +67,12 @@ constexpr int T6_ABUF = T6_NT * T6_TILE;
 constexpr int T6_BBUF = T6_NN * 128;
 constexpr int T6_TPS = T6_W + 8;          // digit-plane row stride (elements)
 // window record: fp16 digit planes [7][4][TPS], double epilogue scales [2][4],
-// mu exponents per 16 l, double2 (a, g) [W + 1] (zero past the window)
+// mu exponents per 16 l, double2 (a, g) [W + 1] (zero past the window), FixCoef [W]
 constexpr int T6_RSC = T6_ND * T6_NO * T6_TPS * 2;
 constexpr int T6_REL = T6_RSC + 2 * T6_NO * 8;
 constexpr int T6_RCO = T6_REL + 32;
-constexpr int T6_RSZ = T6_RCO + (T6_W + 1) * 16;
+constexpr int T6_RFX = T6_RCO + (T6_W + 1) * 16;
+constexpr int T6_RSZ = T6_RFX + T6_W * 16;
 constexpr int T6_OFF_B = 2 * T6_ABUF;
 constexpr int T6_OFF_R = T6_OFF_B + 2 * T6_BBUF;
 constexpr int T6_OFF_BAR = T6_OFF_R + 2 * T6_RSZ;   // full[2], empty[2], record[2]
@@ -135,7 +144,7 @@ __global__ void k_tc64_scale(int L, int s, double2 *__restrict__ b) {
 
 // a_l = alpha_l c_l / c_{l+1}, g_l = gamma_l c_l / c_{l+1} and c_l, rounded once
 __global__ void k_tc64_coef(int L, int s, const double2 *__restrict__ c, double2 *__restrict__ ag,
-                            double *__restrict__ cl) {
+                            double *__restrict__ cl, FixCoef *__restrict__ fx) {
     const int m = blockIdx.y, l = m + blockIdx.x * blockDim.x + threadIdx.x;
     if (l > L) return;
     const long long ix = almidx(L, m, m) - m + l;
@@ -147,6 +156,7 @@ __global__ void k_tc64_coef(int L, int s, const double2 *__restrict__ c, double2
             v.y = dd_div(dd_mul(a, dd{(double)m * s, 0.0}), dd{(double)l * (l + 1), 0.0}).h;
     }
     ag[ix] = v;
+    fx[ix] = fix_coef(v.x, v.y);
     cl[ix] = c[ix].x;
 }
 
@@ -160,6 +170,16 @@ __global__ void k_tc64_chunk_exp(int L, int s, const double *__restrict__ cl, co
     int e = -1000;
     for (int l = lb; l <= min(lb + 15, L); ++l) e = max(e, tc_bound_exp((float)cl[b + l], l));
     eb[8 * (long long)woff[m] + c] = (short)e;
+}
+
+// Es of every order: 2^Es > |mu_l| for all its l
+__global__ void k_tc64_order_exp(int L, int s, const int *__restrict__ woff, const short *__restrict__ eb,
+                                 short *__restrict__ es) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m > L) return;
+    int e = -1000;
+    for (int c = 0, lb = max(m, s); lb <= L; ++c, lb += 16) e = max(e, (int)eb[8 * (long long)woff[m] + c]);
+    es[m] = (short)e;
 }
 
 // Start states: per (m, side, pair) the first chunk of 16 l (from l0) in which
@@ -230,7 +250,9 @@ __global__ void __launch_bounds__(T6_W)
     const int l = wb + i;
     const long long ix = almidx(L, m, m) - m + l;
     double2 *co = reinterpret_cast<double2 *>(R + T6_RCO);
-    co[i] = i < cnt ? ag[ix] : make_double2(0.0, 0.0);
+    const double2 agi = i < cnt ? ag[ix] : make_double2(0.0, 0.0);
+    co[i] = agi;
+    reinterpret_cast<FixCoef *>(R + T6_RFX)[i] = fix_coef(agi.x, agi.y);
     if (i == 0) co[T6_W] = make_double2(0.0, 0.0);
     double v[T6_NO] = {0.0, 0.0, 0.0, 0.0};
     int eb = -1000;
@@ -288,11 +310,11 @@ __global__ void __launch_bounds__(T6_W)
 
 // ---------------------------------------------------------------- synthesis
 template <bool S0>
-__global__ void __launch_bounds__(T6_BLOCK, 1)
+__global__ void __launch_bounds__(T6_BLOCK, 2)
     k_leg_synth_tc64(int L, int spin, const unsigned char *__restrict__ rec, const int *__restrict__ woff,
                      const double2 *__restrict__ lg0, int npairs, const double *__restrict__ px,
                      const RingLog *__restrict__ lsc, const int *__restrict__ prn, const int *__restrict__ prs, const double2 *__restrict__ stv, const short2 *__restrict__ ste,
-                     int st_ld, double2 *__restrict__ H, int ldH, int *status) {
+                     int st_ld, const short *__restrict__ es, double2 *__restrict__ H, int ldH, int *status) {
     constexpr int T = T6_T;
     extern __shared__ __align__(1024) unsigned char sm[];
     uint32_t *s_tm = reinterpret_cast<uint32_t *>(sm + T6_OFF_TM);
@@ -397,6 +419,14 @@ __global__ void __launch_bounds__(T6_BLOCK, 1)
         const int tile = tid >> 7, row = tid & 127;
         const double xs = act ? (side ? -px[p] : px[p]) : 0.0;
         double acc[T6_NO] = {0.0, 0.0, 0.0, 0.0};
+        // fixed point once every ring of the warp is past its turning point (cur, prev then hold U, V)
+        const int Es = es[m];
+        const long long X = fix62(xs, 1);  // Q61
+        const int xh = (int)(X >> 31), xl = (int)X & 0x7FFFFFFF;
+        const bool idle = c_me == TC_NEVER;  // never accumulates: stays zero
+        const long long rnd = idle ? 0 : FIX_ROUND;
+        bool fixed = false;
+        const bool may_fix = __any_sync(0xffffffffu, !idle);
         const uint32_t t_lane = tbase + ((uint32_t)((warp & 3) * 32) << 16) + tile * T6_NN;
         const uint32_t a_row = (uint32_t)tile * T6_TILE + (row >> 3) * T6_SBO + (row & 7) * 16;
         // this thread's B' copy: row n = g NO + o, K-core di = t_{g-di} of output o (28 pairs x 4 outputs)
@@ -427,6 +457,7 @@ __global__ void __launch_bounds__(T6_BLOCK, 1)
             const double *s_sc = reinterpret_cast<const double *>(Rw + T6_RSC);
             const int *s_el = reinterpret_cast<const int *>(Rw + T6_REL);
             const double2 *s_ag = reinterpret_cast<const double2 *>(Rw + T6_RCO);
+            const FixCoef *s_fx = reinterpret_cast<const FixCoef *>(Rw + T6_RFX);
 
             const int nch = (cnt + T6_KC - 1) / T6_KC;
             for (int c = kw == kw0 ? cs0 : 0; c < nch; ++c, ++gc) {
@@ -438,8 +469,42 @@ __global__ void __launch_bounds__(T6_BLOCK, 1)
                 if (b_dst >= 0)
                     *reinterpret_cast<uint4 *>(sB + b_dst) =
                         *reinterpret_cast<const uint4 *>(s_tp + b_src + c * T6_KC);
-                if (live) {
-                    const int nb = 1030 + s_el[c >> 1] - e;  // e < 0: every digit 0
+                const int El = s_el[c >> 1];
+                if (may_fix && !fixed) {
+                    const double2 a = s_ag[c * T6_KC];
+                    fixed = __all_sync(0xffffffffu, idle || (live && fix_ready(cur, prev, e, a.x, a.y, xs, Es, El)));
+                    if (fixed) {
+                        cur = __longlong_as_double(idle ? 0 : fix62(cur, Es));
+                        prev = __longlong_as_double(idle ? 0 : fix62(prev, Es));
+                    }
+                }
+                if (fixed) {
+                    const int sh = 7 + El - Es;
+                    long long U = __double_as_longlong(cur), V = __double_as_longlong(prev);
+                    uint32_t pk[T6_ND][4];
+#pragma unroll
+                    for (int j2 = 0; j2 < 4; ++j2) {
+                        const FixCoef q0 = s_fx[c * T6_KC + 2 * j2], q1 = s_fx[c * T6_KC + 2 * j2 + 1];
+                        const unsigned long long w0 = (unsigned long long)(U >> sh) + FIX_BIAS;
+                        fix_step(q0, xh, xl, rnd, U, V);
+                        const unsigned long long w1 = (unsigned long long)(U >> sh) + FIX_BIAS;
+                        fix_step(q1, xh, xl, rnd, U, V);
+                        pk[0][j2] = digit_pair<0>(w0, w1);
+                        pk[1][j2] = digit_pair<1>(w0, w1);
+                        pk[2][j2] = digit_pair<2>(w0, w1);
+                        pk[3][j2] = digit_pair<3>(w0, w1);
+                        pk[4][j2] = digit_pair<4>(w0, w1);
+                        pk[5][j2] = digit_pair<5>(w0, w1);
+                        pk[6][j2] = digit_pair<6>(w0, w1);
+                    }
+                    cur = __longlong_as_double(U);
+                    prev = __longlong_as_double(V);
+#pragma unroll
+                    for (int k = 0; k < T6_ND; ++k)
+                        *reinterpret_cast<uint4 *>(sA + a_row + k * 128) =
+                            make_uint4(pk[k][0], pk[k][1], pk[k][2], pk[k][3]);
+                } else if (live) {
+                    const int nb = 1030 + El - e;  // e < 0: every digit 0
                     uint32_t pk[T6_ND][4];
 #pragma unroll
                     for (int j2 = 0; j2 < 4; ++j2) {
@@ -563,9 +628,11 @@ static size_t tc64_layout(cunusht_plan_s *P, char *base, size_t &nrec) {
         nrec = std::max(nrec, w);
         take(P->d_t6_ag[s], P->nalm_tab);
         take(P->d_t6_cl[s], P->nalm_tab);
+        take(P->d_t6_fx[s], P->nalm_tab);
         take(P->d_t6_lg0[s], L + 1);
         take(P->d_t6_eb[s], 8 * w);
         take(P->d_t6_woff[s], L + 2);
+        take(P->d_t6_es[s], L + 1);
     }
     take(P->d_t6_rec, nrec * T6_RSZ);
     for (int g = 0; g < 2; ++g) {
@@ -584,7 +651,7 @@ static int tc64_tables(cunusht_plan_s *P, int s, double2 *cdd) {
     const dim3 grid((L + 256) / 256, L + 1);
     k_tc64_beta<<<grid, 256>>>(L, s, cdd);
     k_tc64_scale<<<(L + 32) / 32, 32>>>(L, s, cdd);
-    k_tc64_coef<<<grid, 256>>>(L, s, cdd, P->d_t6_ag[s], P->d_t6_cl[s]);
+    k_tc64_coef<<<grid, 256>>>(L, s, cdd, P->d_t6_ag[s], P->d_t6_cl[s], P->d_t6_fx[s]);
     CU_LAUNCH_CHECK();
     // log2 of the start's normalisation sqrt((2 l0 + 1) / (4 pi) (2 l0)! / ((m + s)! |m - s|!)), l0 = max(m, s)
     std::vector<double2> lg(L + 1);
@@ -602,6 +669,7 @@ static int tc64_tables(cunusht_plan_s *P, int s, double2 *cdd) {
     CU_TRY(cudaMemcpy(P->d_t6_lg0[s], lg.data(), lg.size() * sizeof(double2), cudaMemcpyHostToDevice));
     CU_TRY(cudaMemcpy(P->d_t6_woff[s], wo.data(), wo.size() * sizeof(int), cudaMemcpyHostToDevice));
     k_tc64_chunk_exp<<<dim3((L / 16 + 64) / 64, L + 1), 64>>>(L, s, P->d_t6_cl[s], P->d_t6_woff[s], P->d_t6_eb[s]);
+    k_tc64_order_exp<<<(L + 64) / 64, 64>>>(L, s, P->d_t6_woff[s], P->d_t6_eb[s], P->d_t6_es[s]);
     CU_LAUNCH_CHECK();
     return CUNUSHT_OK;
 }
@@ -657,7 +725,7 @@ int leg_synth_tc64(const cunusht_plan_s *P, int npairs, const double *x, const d
         if (stv) ++stv, ++ste;
         --npairs;
     }
-    const int per = spin == 0 ? T6_T : T6_T / 2, tail = npairs % per;
+    const int per = spin == 0 ? T6_T : T6_T / 2, tail = npairs % (spin == 0 ? 512 : 256);
     const int ntc = (npairs > per && tail < T6_MIN_TAIL) ? npairs - tail : npairs;
     k_tc64_records<<<dim3((L - spin + T6_W) / T6_W, P->mmax + 1), T6_W, 0, st>>>(
         L, spin, G, C, lf, P->d_t6_ag[spin], P->d_t6_cl[spin], P->d_t6_woff[spin], P->d_t6_rec);
@@ -665,8 +733,8 @@ int leg_synth_tc64(const cunusht_plan_s *P, int npairs, const double *x, const d
     auto launch = [&](auto kern) {
         CU_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T6_BYTES));
         kern<<<dim3((ntc + per - 1) / per, P->mmax + 1), T6_BLOCK, T6_BYTES, st>>>(
-            L, spin, P->d_t6_rec, P->d_t6_woff[spin], P->d_t6_lg0[spin], ntc, x, lsc, rn, rs, stv, ste, st_ld, H, ld,
-            P->d_status);
+            L, spin, P->d_t6_rec, P->d_t6_woff[spin], P->d_t6_lg0[spin], ntc, x, lsc, rn, rs, stv, ste, st_ld,
+            P->d_t6_es[spin], H, ld, P->d_status);
         CU_LAUNCH_CHECK();
         return CUNUSHT_OK;
     };

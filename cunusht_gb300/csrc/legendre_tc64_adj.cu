@@ -58,7 +58,8 @@ __device__ __forceinline__ long long shfl_xor_ll(long long v, int mask) { return
 template <bool S0>
 __global__ void __launch_bounds__(A6_THREADS, 1)
     k_leg_adj_tc64(int L, int spin, int ncomp, const double2 *__restrict__ H, int ldH, const double *__restrict__ lfac,
-                   const double2 *__restrict__ ag, const double *__restrict__ cl, const short *__restrict__ eb,
+                   const double2 *__restrict__ ag, const FixCoef *__restrict__ fx, const double *__restrict__ cl,
+                   const short *__restrict__ eb, const short *__restrict__ es,
                    const int *__restrict__ woff, const double2 *__restrict__ lg0, int npairs,
                    const double *__restrict__ px, const RingLog *__restrict__ lsc, const int *__restrict__ prn,
                    const int *__restrict__ prs, const double2 *__restrict__ stv, const short2 *__restrict__ ste,
@@ -224,14 +225,16 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
 #pragma unroll
             for (int q = 0; q < 8; ++q) hi[q] = lo[q] = 0;
             const uint32_t ta = tbase + tb * 128 + 8 * eh;
+            float v[A6_ND][8];  // all loads in flight before the one wait
+#pragma unroll
+            for (int i = 0; i < A6_ND; ++i) tmem_ld8_async(ta + i * A6_KC, v[i]);
+            tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < A6_ND; ++i) {
-                float v[8];
-                tmem_ld8(ta + i * A6_KC, v);
                 const bool ih = i + j <= 3, il = !ih && i + j <= 6;
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    const int d = (int)v[q];
+                    const int d = (int)tmem_keep(v[i][q]);
                     if (ih) hi[q] = (hi[q] << 8) + d;
                     if (il) lo[q] = (lo[q] << 8) + d;
                 }
@@ -277,6 +280,14 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
     } else {
         // ---------------- ring warps
         const double xs = act ? (side ? -px[p] : px[p]) : 0.0;
+        // fixed point once every ring of the warp is past its turning point (rec64.cuh)
+        const int Es = es[m];
+        const long long XQ = fix62(xs, 1);  // Q61
+        const int xh = (int)(XQ >> 31), xl = (int)XQ & 0x7FFFFFFF;
+        const bool idle = c_me == TC_NEVER;
+        const long long rnd = idle ? 0 : FIX_ROUND;
+        bool fixed = false;
+        const bool may_fix = __any_sync(0xffffffffu, !idle);
         const uint32_t boff = (rid >> 3) * A6_B_LBO + (rid & 7) * 16;
         int gc = 0, bad = 0;
         for (int lb = lstart; lb <= L; lb += A6_KC, ++gc) {
@@ -285,10 +296,49 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
             bad = __any_sync(0xffffffffu, bad | *s_bad);
             if (bad) break;
             unsigned char *sB = sm + A6_OFF_B + buf * A6_BBUF + boff;
-            if (ck >= c_me) {  // before its first chunk a ring holds its table state and writes zero digits
+            const bool live = ck >= c_me;  // before its first chunk a ring holds its table state and writes zero digits
+            const int El = ebm[ck];
+            if (may_fix && !fixed) {
+                const double2 a = __ldg(ag + b + lb);
+                fixed = __all_sync(0xffffffffu, idle || (live && fix_ready(cur, prev, e, a.x, a.y, xs, Es, El)));
+                if (fixed) {
+                    cur = __longlong_as_double(idle ? 0 : fix62(cur, Es));
+                    prev = __longlong_as_double(idle ? 0 : fix62(prev, Es));
+                }
+            }
+            if (fixed) {
+                const int sh = 7 + El - Es;
+                long long U = __double_as_longlong(cur), V = __double_as_longlong(prev);
 #pragma unroll
                 for (int lh = 0; lh < 2; ++lh) {
-                    const int nb = 1030 + ebm[ck] - e;  // e < 0: every digit 0
+                    uint32_t pk[A6_ND][4];
+#pragma unroll
+                    for (int j2 = 0; j2 < 4; ++j2) {
+                        const int l = lb + 8 * lh + 2 * j2;
+                        const FixCoef q0 = fix_load(fx + b + min(l, L)), q1 = fix_load(fx + b + min(l + 1, L));
+                        const unsigned long long w0 = (unsigned long long)(U >> sh) + FIX_BIAS;
+                        fix_step(q0, xh, xl, rnd, U, V);
+                        const unsigned long long w1 = (unsigned long long)(U >> sh) + FIX_BIAS;
+                        fix_step(q1, xh, xl, rnd, U, V);
+                        pk[0][j2] = digit_pair<0>(w0, w1);
+                        pk[1][j2] = digit_pair<1>(w0, w1);
+                        pk[2][j2] = digit_pair<2>(w0, w1);
+                        pk[3][j2] = digit_pair<3>(w0, w1);
+                        pk[4][j2] = digit_pair<4>(w0, w1);
+                        pk[5][j2] = digit_pair<5>(w0, w1);
+                        pk[6][j2] = digit_pair<6>(w0, w1);
+                    }
+#pragma unroll
+                    for (int k = 0; k < A6_ND; ++k)
+                        *reinterpret_cast<uint4 *>(sB + (2 * k + lh) * A6_B_SBO) =
+                            make_uint4(pk[k][0], pk[k][1], pk[k][2], pk[k][3]);
+                }
+                cur = __longlong_as_double(U);
+                prev = __longlong_as_double(V);
+            } else if (live) {
+#pragma unroll
+                for (int lh = 0; lh < 2; ++lh) {
+                    const int nb = 1030 + El - e;  // e < 0: every digit 0
                     uint32_t pk[A6_ND][4];
 #pragma unroll
                     for (int j2 = 0; j2 < 4; ++j2) {
@@ -361,8 +411,8 @@ int leg_adjoint_tc64(const cunusht_plan_s *P, int npairs, const double *x, const
     auto launch = [&](auto kern) {
         CU_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, A6_BYTES));
         kern<<<dim3((ntc + per - 1) / per, P->mmax + 1), A6_THREADS, A6_BYTES, st>>>(
-            L, spin, ncomp, H, ld, lf, P->d_t6_ag[spin], P->d_t6_cl[spin], P->d_t6_eb[spin], P->d_t6_woff[spin],
-            P->d_t6_lg0[spin], ntc, x, lsc, rn, rs, stv, ste, st_ld, (double *)G, (double *)C, P->d_status);
+            L, spin, ncomp, H, ld, lf, P->d_t6_ag[spin], P->d_t6_fx[spin], P->d_t6_cl[spin], P->d_t6_eb[spin],
+            P->d_t6_es[spin], P->d_t6_woff[spin], P->d_t6_lg0[spin], ntc, x, lsc, rn, rs, stv, ste, st_ld, (double *)G, (double *)C, P->d_status);
         CU_LAUNCH_CHECK();
         return CUNUSHT_OK;
     };

@@ -141,6 +141,59 @@ __device__ __forceinline__ unsigned long long fix55_biased(double v, int nb) {
     return ((M >> n) ^ (unsigned long long)s) + (FIX_BIAS - (unsigned long long)s);
 }
 
+// ---------------------------------------------------------------- fixed-point recursion
+// Past its turning point a ring's mu stays within a few binary orders of its
+// bound, so the recursion can run in 64-bit fixed point on the integer pipes:
+// U = mu 2^(62 - Es) with 2^Es > |mu| up to lmax, x in Q61, a in Q58 (a < 8), g
+// and t = a x + g in Q60 (|t| < 4).  Products of 31-bit halves (three
+// IMAD.WIDE each; the low x low term enters by its mean) leave an error of
+// about one unit per step, 2^-62 of the bound or 2^-56 of the amplitude at
+// lmax 2047, against 2^-54 of an FP64 step.  About 30 integer instructions per
+// step and ring, digits included, at 64 lanes per SM and clock, in place of
+// two FP64 instructions at 2.
+struct alignas(16) FixCoef {
+    int ah, al;    // a 2^58 = ah 2^31 + al
+    long long g;   // g 2^60
+};
+__device__ __forceinline__ FixCoef fix_load(const FixCoef *p) {
+    const int4 q = __ldg(reinterpret_cast<const int4 *>(p));
+    return FixCoef{q.x, q.y, (long long)(((unsigned long long)(unsigned)q.w << 32) | (unsigned)q.z)};
+}
+// v 2^(62 - Eb) for |v| < 2^Eb, truncated
+__device__ __forceinline__ long long fix62(double v, int Eb) {
+    const int hi = __double2hiint(v);
+    const unsigned n = min((unsigned)(1023 + Eb - ((hi >> 20) & 0x7FF)), 63u);  // >= 1
+    const unsigned long long M =
+        (((unsigned long long)(((unsigned)hi & 0xFFFFFu) | 0x100000u) << 32) | (unsigned)__double2loint(v)) << 10;
+    const long long s = (long long)(hi >> 31);
+    return (long long)((M >> n) ^ (unsigned long long)s) - s;
+}
+__device__ __forceinline__ FixCoef fix_coef(double a, double g) {
+    const long long A = a < 8.0 ? fix62(a, 4) : 0;  // Q58
+    return FixCoef{(int)(A >> 31), (int)(A & 0x7FFFFFFF), fabs(g) < 4.0 ? fix62(g, 2) : 0};
+}
+// rnd: FIX_ROUND, or 0 for a ring that stays zero (a rounding constant would grow where |t| > 2)
+constexpr long long FIX_ROUND = (1LL << 28) + (1LL << 29);
+__device__ __forceinline__ void fix_step(const FixCoef q, int xh, int xl, long long rnd, long long &U, long long &V) {
+    const long long p = (long long)q.ah * xh;
+    const long long cr = (long long)q.al * xh + ((long long)q.ah * xl + rnd);
+    const long long T = (q.g + (p * 8)) + (cr >> 28);
+    const int th = (int)(T >> 31), tl = (int)T & 0x7FFFFFFF, uh = (int)(U >> 31), ul = (int)U & 0x7FFFFFFF;
+    const long long p2 = (long long)uh * th;
+    const long long c2 = (long long)ul * th + ((long long)uh * tl + rnd);
+    // modulo 2^64: t U may pass 2^63, mu_{l+1} does not
+    const unsigned long long N = (((unsigned long long)p2 << 2) - (unsigned long long)V) + (unsigned long long)(c2 >> 29);
+    V = U;
+    U = (long long)N;
+}
+// Whether a ring may go over to fixed point at a chunk with digit exponent El:
+// |mu| or |previous mu| at least 2^(Es - 9), a and |t| small enough from here
+// on (both fall towards 2 and 2 |x|), the digits a right shift of U by 0 .. 7.
+__device__ __forceinline__ bool fix_ready(double cur, double prev, int e, double a, double g, double x, int Es, int El) {
+    const int ec = (__double2hiint(cur) >> 20) & 0x7FF, ep = (__double2hiint(prev) >> 20) & 0x7FF;
+    return e == 0 && max(ec, ep) - 1023 >= Es - 9 && a < 7.5 && fabs(fma(a, x, g)) < 3.0 && El + 7 >= Es;
+}
+
 // digit K of the biased words of two values as packed fp16 (a low, b high):
 // the bit pattern 0x6400 | (digit + 128) is 1024 + (digit + 128); minus 1152, exact
 template <int K> __device__ __forceinline__ uint32_t digit_pair(unsigned long long a, unsigned long long b) {

@@ -168,6 +168,20 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// tmem_ld8 in two parts: several loads may be in flight before tmem_ld_wait, and the values are
+// read through tmem_keep after it (which keeps the compiler from moving their use before the wait)
+__device__ __forceinline__ void tmem_ld8_async(uint32_t taddr, float (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ float tmem_keep(float v) {
+    asm volatile("" : "+f"(v));
+    return v;
+}
+
 // ---------------------------------------------------------------- digit split
 // x = (h + l) sc for a power of two sc (|h sc| <= 128) as d0 + d1/256 +
 // d2/256^2 + d3/256^3 + O(2^-25), integer digits |d_i| <= 128.  The integer
