@@ -1306,6 +1306,7 @@ int ring_synth(const cunusht_plan_s *P, int spin, const double2 *Hgl, double *ou
 
 int ring_adjoint(const cunusht_plan_s *P, int spin, const double *in0, const double *in1,
                  double2 *Hgl, cudaStream_t st, const double *wring) {
+    if (ring_mr_available(P)) return ring_adjoint_mr(P, spin, in0, in1, Hgl, st, wring);
     size_t sm = fft_smem_bytes(ring_buffer_len(P), false);
     RC_TRY(set_smem(k_ring_adj, sm));
     const RingCls rc = ring_cls_of(P);

@@ -15,6 +15,9 @@ bool ring_mr_available(const cunusht_plan_s *P);
 int ring_synth_mr_batch(const cunusht_plan_s *P, int nreq, int spin, const double2 *Hgl, long long hbs, double *out0,
                         double *out1, long long obs, cudaStream_t st);
 
+int ring_adjoint_mr(const cunusht_plan_s *P, int spin, const double *in0, const double *in1, double2 *Hgl,
+                    cudaStream_t st, const double *wring);
+
 // capi.cu: Gauss-Legendre nodes x (descending cos theta) and weights, Newton iteration
 void gauss_legendre(int n, std::vector<double> &x, std::vector<double> &w);
 
