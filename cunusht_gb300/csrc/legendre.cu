@@ -1099,12 +1099,13 @@ int leg_synth_spin_df_pairs(const cunusht_plan_s *P, int nb, int npairs, const d
 }
 
 // FP64 plans go to the tensor cores unless the work is a few microseconds:
-// below lmax 56 a spin-0 transform is quicker in the one launch of the
-// CUDA-core kernel than in records, pole pair and main kernel (synthesis lmax
-// 31: 31 against 35 us, 47: 33 against 37, 63: 39 against 37; spin 2 at 31: 43
+// below lmax 96 a spin-0 transform takes less device time than the launches
+// of a call (about 65 us), and the CUDA-core kernel is one launch where
+// records, pole pair and main kernel are three (back to back: synthesis lmax
+// 31 31 against 35 us, 63 39 against 37, 127 60 against 41; spin 2 at 31 43
 // against 36).
 static bool f64_tensor_cores(const cunusht_plan_s *P, int spin) {
-    return P->use_tc && P->d_t6_ag[spin] && (spin > 0 || P->lmax >= 56);
+    return P->use_tc && P->d_t6_ag[spin] && (spin > 0 || P->lmax >= 96);
 }
 
 // nreq requests (alm at G + r * astride, columns at H + r * hstride); the
