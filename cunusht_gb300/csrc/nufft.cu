@@ -320,13 +320,37 @@ __device__ __forceinline__ double f2d_exact_int(float f) {
     return __longlong_as_double((long long)bits);
 }
 
+// x - c of a Kahan pair as one double, on the integer pipe: -c, rounded to
+// units of 2^-52 of x's binade, is added to the shifted mantissa of x.  Refused
+// (false) where that leaves the binade, where c is not small against x, and
+// for zero, tiny, infinite and NaN x; the two parts are then added one by one.
+__device__ __forceinline__ bool kahan_f64_int(float x, float c, double &v) {
+    const unsigned u = __float_as_uint(x);
+    const unsigned ex = (u >> 23) & 0xffu;
+    const float unit = __uint_as_float((306u - ex) << 23);  // 2^(52 - e), e = ex - 127
+    const float k = __uint_as_float(__float_as_uint(c) ^ ~u & 0x80000000u) * unit;
+    const unsigned hi = (ex + 896u) << 20;
+    const unsigned long long bits = (((unsigned long long)hi) << 32 | (unsigned long long)(u & 0x7fffffu) << 29) +
+                                    (unsigned long long)(long long)__float2int_rn(k);
+    v = __longlong_as_double((long long)(bits | (unsigned long long)(u & 0x80000000u) << 32));
+    return ex - 52u <= 202u && fabsf(k) < 1073741824.f && ((unsigned)(bits >> 32) & 0x7ff00000u) == hi;
+}
+
 // Mixed-precision variant: kernel weights in FP32 from the FP64 tap offset
 // split into hi + lo floats (as k_interp_mixed), FP32 products, global
-// accumulation in the grid's type TG.  FP64 grid (eps <= 1e-6):
-// Kahan-compensated FP32 strip sums, each added as two exact FP64 atomics.
-// FP32 grid (eps > 1e-6): plain FP32 strip sums (half the shared memory, so
-// twice the resident blocks) and one FP32 atomic per strip cell.  The FP64 variant is bound by its FP64 exponentials and
-// products (GB300 runs FP64 at about 1/80 of the FP32 rate).
+// accumulation in the grid's type TG.
+// FP64 grid (eps <= 1e-6): Kahan-compensated FP32 strip sums, each cell added
+// as one FP64 atomic.  The strip holds one component at a time, which keeps
+// six blocks on an SM instead of three: the taps are a serial
+// read-modify-write, and 12 warps per SM left 60 % of the issue slots empty.
+// Its columns are stored evens first, odds second: neighbouring points lie
+// about two fine cells apart (the grid is oversampled by two), so one tap of
+// 32 lanes reads 32 consecutive cells and not every second one.  Adding
+// sum and compensation as one FP64 value halves the atomics.  Four spin-2 maps
+// of 8.4 M points, w = 9: 13.9 -> 10.6 ms (issue slots 41 -> 63 % used, shared
+// memory 74 %).
+// FP32 grid (eps > 1e-6): plain FP32 strip sums of both components and one
+// FP32 atomic per strip cell.
 template <typename TG, bool CPLX, int W>
 __global__ void __launch_bounds__(SPW_WARPS * 32)
     k_spread_warp_mixed(TG *__restrict__ U, int nrows, int Npf, int Ntf, int n_lo, int w, float beta,
@@ -339,7 +363,7 @@ __global__ void __launch_bounds__(SPW_WARPS * 32)
     constexpr bool KAHAN = std::is_same<TG, double>::value;
     using SE = typename std::conditional<KAHAN, float2, float>::type;  // (sum, compensation) or sum
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    SE *strip = reinterpret_cast<SE *>(smem_raw) + (size_t)wid * SR * SC * NC;
+    SE *strip = reinterpret_cast<SE *>(smem_raw) + (size_t)wid * SR * (KAHAN ? SC + 1 : SC * NC);
     const int E = Ufix ? fix_exp(vmax[blockIdx.y], lgn) : 0;
     if (Ufix) Ufix += blockIdx.y * ubs;
     U += blockIdx.y * ubs;  // request of a batch
@@ -428,23 +452,81 @@ __global__ void __launch_bounds__(SPW_WARPS * 32)
         }
         return;
     }
-    for (int i = lane; i < nr * ncl * NC; i += 32) strip[i] = SE{};
-    __syncwarp();
     const int key = act ? (pc.r0 - rmin) * SC + (pc.p0 - pmin) : -1 - lane;
     const unsigned peers = __match_any_sync(0xffffffffu, key);
     const int myrank = __popc(peers & ((1u << lane) - 1u));
     const int nround = __reduce_max_sync(0xffffffffu, act ? myrank : 0) + 1;
-    const int base = (pc.r0 - rmin) * ncl + (pc.p0 - pmin);
-    for (int rd = 0; rd < nround; ++rd) {
-        const bool go = act && myrank == rd;
+    if constexpr (KAHAN) {
+        const int half = (ncl + 1) >> 1, pitch = 2 * half;
+        const int rl = pc.r0 - rmin, cl = pc.p0 - pmin;
+        const int q32 = 32 / ncl, r32 = 32 - q32 * ncl;
+        // taps 0, 2, ... of a row start at the first, taps 1, 3, ... at the second
+        SE *const row_e = strip + rl * pitch + (cl & 1) * half + (cl >> 1);
+        SE *const row_o = strip + rl * pitch + (~cl & 1) * half + ((cl + 1) >> 1);
 #pragma unroll 1
-        for (int a = 0; a < W; ++a) {
-            // row factor kt[a] * value as a double-float (FP32 TwoProduct on
-            // the split value): each tap product then carries one FP32 rounding
-            const float frh = kt[a] * vrh, frl = fmaf(kt[a], vrh, -frh) + kt[a] * vrl;
-            const float fih = kt[a] * vih, fil = fmaf(kt[a], vih, -fih) + kt[a] * vil;
-            SE *row = strip + (size_t)(base + a * ncl) * NC;
-            if constexpr (!KAHAN) {
+        for (int q = 0; q < NC; ++q) {
+            const float vh = q ? vih : vrh, vl = q ? vil : vrl;
+            for (int i = lane; i < nr * pitch; i += 32) strip[i] = SE{};
+            __syncwarp();
+            for (int rd = 0; rd < nround; ++rd) {
+                const bool go = act && myrank == rd;
+#pragma unroll
+                for (int a = 0; a < W; ++a) {
+                    // row factor kt[a] * value as a double-float (FP32 TwoProduct on
+                    // the split value): each tap product then carries one FP32 rounding
+                    const float fh = kt[a] * vh, fl = fmaf(kt[a], vh, -fh) + kt[a] * vl;
+                    SE *re = row_e + a * pitch, *ro = row_o + a * pitch;
+#pragma unroll
+                    for (int b = 0; b < W; ++b) {
+                        if (go) {
+                            // Kahan: sum = x, comp = c; value = x - c
+                            SE *cp = (b & 1 ? ro : re) + (b >> 1);
+                            const float2 t = *cp;
+                            const float y = fmaf(kp[b], fh, kp[b] * fl) - t.y;
+                            const float s2 = t.x + y;
+                            *cp = make_float2(s2, (s2 - t.x) - y);
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+            int lr = lane / ncl, lc = lane - lr * ncl;
+            for (int i = lane; i < nr * ncl; i += 32) {
+                int c = pmin + lc;
+                c = c < 0 ? c + Npf : (c >= Npf ? c - Npf : c);
+                const long long ci = ((long long)(rmin + lr) * Npf + c) * NC + q;
+                const float2 v = strip[lr * pitch + (lc & 1) * half + (lc >> 1)];
+                double d;
+                if (Ufix) {
+                    if (v.x != 0.f || v.y != 0.f)
+                        atomicAdd(Ufix + ci, (unsigned long long)(to_fix(v.x, E) - to_fix(v.y, E)));
+                } else if (kahan_f64_int(v.x, v.y, d)) {
+                    atomicAdd(U + ci, d);
+                } else {
+                    if (v.x != 0.f) atomicAdd(U + ci, f2d_exact_int(v.x));
+                    if (v.y != 0.f) atomicAdd(U + ci, f2d_exact_int(-v.y));
+                }
+                lr += q32;
+                lc += r32;
+                if (lc >= ncl) {
+                    lc -= ncl;
+                    ++lr;
+                }
+            }
+            __syncwarp();
+        }
+        return;
+    } else {
+        for (int i = lane; i < nr * ncl * NC; i += 32) strip[i] = SE{};
+        __syncwarp();
+        const int base = (pc.r0 - rmin) * ncl + (pc.p0 - pmin);
+        for (int rd = 0; rd < nround; ++rd) {
+            const bool go = act && myrank == rd;
+#pragma unroll 1
+            for (int a = 0; a < W; ++a) {
+                const float frh = kt[a] * vrh, frl = fmaf(kt[a], vrh, -frh) + kt[a] * vrl;
+                const float fih = kt[a] * vih, fil = fmaf(kt[a], vih, -fih) + kt[a] * vil;
+                SE *row = strip + (size_t)(base + a * ncl) * NC;
 #pragma unroll
                 for (int b = 0; b < W; ++b) {
                     if (go) {
@@ -453,53 +535,19 @@ __global__ void __launch_bounds__(SPW_WARPS * 32)
                     }
                     __syncwarp();
                 }
-            } else {
-#pragma unroll
-                for (int b = 0; b < W; ++b) {
-                    if (go) {
-                        // Kahan: sum = x, comp = c; value = x - c
-                        float2 t = row[b * NC];
-                        float y = fmaf(kp[b], frh, kp[b] * frl) - t.y;
-                        float s2 = t.x + y;
-                        row[b * NC] = make_float2(s2, (s2 - t.x) - y);
-                        if constexpr (CPLX) {
-                            t = row[b * NC + 1];
-                            y = fmaf(kp[b], fih, kp[b] * fil) - t.y;
-                            s2 = t.x + y;
-                            row[b * NC + 1] = make_float2(s2, (s2 - t.x) - y);
-                        }
-                    }
-                    __syncwarp();
-                }
             }
         }
-    }
-    __syncwarp();
-    for (int i = lane; i < nr * ncl; i += 32) {
-        const int lr = i / ncl, lc = i - lr * ncl;
-        int c = pmin + lc;
-        c = c < 0 ? c + Npf : (c >= Npf ? c - Npf : c);
-        const long long ci = ((long long)(rmin + lr) * Npf + c) * NC;
-        TG *cell = U + ci;
+        for (int i = lane; i < nr * ncl; i += 32) {
+            const int lr = i / ncl, lc = i - lr * ncl;
+            int c = pmin + lc;
+            c = c < 0 ? c + Npf : (c >= Npf ? c - Npf : c);
+            const long long ci = ((long long)(rmin + lr) * Npf + c) * NC;
 #pragma unroll
-        for (int q = 0; q < NC; ++q) {
-            // Kahan value x - c as two exact FP64 atomic adds (the additions
-            // happen in L2, the conversions on the integer pipe), or as one
-            // FP32 atomic add of x - c into an FP32 grid
-            if constexpr (KAHAN) {
-                const float2 v = strip[i * NC + q];
-                if (Ufix) {
-                    if (v.x != 0.f || v.y != 0.f)
-                        atomicAdd(Ufix + ci + q, (unsigned long long)(to_fix(v.x, E) - to_fix(v.y, E)));
-                    continue;
-                }
-                if (v.x != 0.f) atomicAdd(cell + q, f2d_exact_int(v.x));
-                if (v.y != 0.f) atomicAdd(cell + q, -f2d_exact_int(v.y));
-            } else {
+            for (int q = 0; q < NC; ++q) {
                 const float v = strip[i * NC + q];
                 if (v == 0.f) continue;
                 if (Ufix) atomicAdd(Ufix + ci + q, (unsigned long long)to_fix(v, E));
-                else atomicAdd(cell + q, v);
+                else atomicAdd(U + ci + q, v);
             }
         }
     }
@@ -512,7 +560,9 @@ static int launch_spread_warp_mixed(const cunusht_plan_s *P, int nreq, TG *U, lo
     int lgn = 0;
     while ((1LL << lgn) < npts + 1) ++lgn;
     const int SR = P->w + 4, SC = 80 + P->w;
-    const size_t sm = (size_t)SPW_WARPS * SR * SC * (CPLX ? 2 : 1) * (std::is_same<TG, double>::value ? 8 : 4);
+    // FP64 grid: (sum, compensation) of one component, columns rounded up to even
+    const size_t sm =
+        (size_t)SPW_WARPS * SR * (std::is_same<TG, double>::value ? (SC + 1) * 8 : SC * (CPLX ? 8 : 4));
     const long long nwarps = (npts + 31) / 32;
     const unsigned nb = (unsigned)((nwarps + SPW_WARPS - 1) / SPW_WARPS);
     cudaError_t e = cudaSuccess;

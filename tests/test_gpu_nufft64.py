@@ -60,3 +60,28 @@ def test_pointing_series_and_large_angles(built_lib, rms):
     dg = np.remainder(gam - g + np.pi, 2 * np.pi) - np.pi
     # the two arctangents of the reference formula cancel where gamma is small
     assert np.max(np.abs(dg) * np.sin(th)) < 32 * ulp
+
+
+@pytest.mark.parametrize("spin", [0, 2])
+@pytest.mark.parametrize("eps", [1e-6, 1e-7])
+@pytest.mark.parametrize("step", [0.0, 0.7, 1.0, 2.0, 2.6])
+def test_mixed_strip_spreading(built_lib, eps, spin, step):
+    """Strips of a mixed plan with an FP64 grid: neighbours ``step`` fine cells apart (repeated
+    points, odd and even columns, the wrap of the longitude), a partial last warp and values of
+    very different size, zero and both signs included (every way a strip cell is added to the grid).
+
+    Tolerance: eps, and four roundings of FP32 (the two weights, their products)."""
+    import cunusht_gb300 as cu
+    lmax, n = 24, 32 * 9 + 5
+    rng = np.random.default_rng(12)
+    k = np.arange(n)
+    th = 1.1 + 0.01 * (k // 96) + 0.002 * np.sin(k)
+    ph = np.remainder(6.2 + k * step * 2 * np.pi / 108, 2 * np.pi)
+    v = rng.standard_normal((2, n) if spin else n)
+    v = v * 10.0 ** rng.integers(-14, 1, v.shape)
+    v[..., 5::17] = 0.0
+    t = cu.get_transformer("GPU")(("gl", {"lmax": lmax}), nuFFTtype=2, epsilon=eps, precision="mixed")
+    loc = torch.as_tensor(np.stack([th, ph], 1), device="cuda")
+    got = t.nusht2d1(lmax, lmax, torch.as_tensor(v, device="cuda"), loc, spin=spin).cpu().numpy()
+    ref = orc.adjoint_synth_points(lmax, spin, v, th, ph)
+    assert np.linalg.norm(got - ref) <= (eps + 4 * 2.0 ** -24) * np.linalg.norm(ref)
