@@ -189,16 +189,20 @@ __device__ __forceinline__ void fft_pass16(cplx<T> *buf, int N, int Ns, int dir,
         const int tstep = M / (Ns * 16);
         const int lq = __ffs(M) - 3;  // log2(M / 4)
         const int k = j & (Ns - 1), t1 = k * tstep;
+        C w4[3];  // w^(4 a k), shared by the four butterflies
+        if (Ns > 1) {
+#pragma unroll
+            for (int a = 1; a < 4; ++a) {
+                w4[a - 1] = tw_quarter<T>(stw, 4 * a * t1, lq);
+                if (dir > 0) w4[a - 1].y = -w4[a - 1].y;
+            }
+        }
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             C *u = v + 4 * b;
             if (Ns > 1) {
 #pragma unroll
-                for (int a = 1; a < 4; ++a) {
-                    C w = tw_quarter<T>(stw, 4 * a * t1, lq);
-                    if (dir > 0) w.y = -w.y;
-                    u[a] = cmul(u[a], w);
-                }
+                for (int a = 1; a < 4; ++a) u[a] = cmul(u[a], w4[a - 1]);
             }
             dft4(u[0], u[1], u[2], u[3], dir);  // u[q]: frequency q over a
             asm volatile("" ::: "memory");
@@ -207,6 +211,7 @@ __device__ __forceinline__ void fft_pass16(cplx<T> *buf, int N, int Ns, int dir,
         for (int q = 0; q < 4; ++q) {
 #pragma unroll
             for (int b = 1; b < 4; ++b) {
+                if (q == 0 && Ns == 1) continue;  // a factor of 1
                 // w^(b k) e^{-2 pi i b q / 16}: table index b (t1 + q M / 16)
                 C w = tw_quarter<T>(stw, b * (t1 + q * (M >> 4)), lq);
                 if (dir > 0) w.y = -w.y;
@@ -216,6 +221,63 @@ __device__ __forceinline__ void fft_pass16(cplx<T> *buf, int N, int Ns, int dir,
             const int idxD = (j - k) * 16 + k;
 #pragma unroll
             for (int p = 0; p < 4; ++p) buf[idxD + (q + 4 * p) * Ns] = v[4 * p + q];
+            asm volatile("" ::: "memory");
+        }
+    }
+    __syncthreads();
+}
+
+// The radix-4 and the radix-2 pass that passes of 16 leave of three factors of
+// two, again as one round trip: 16 elements per thread in two groups of 8.
+// Element r = 2 a + b: radix-4 over a with w^(2 a k), the factors
+// e^{dir 2 pi i b q / 8} w^(b k), radix-2 over b, which gives output q + 4 p.  As
+// in fft_pass16 the operations are those of the single passes.
+template <typename T>
+__device__ __forceinline__ void fft_pass8(cplx<T> *buf, int N, int Ns, int dir, const cplx<T> *__restrict__ stw, int M,
+                                          int nthr) {
+    using C = cplx<T>;
+    const int nb = N / 8;  // == 2 nthr
+    const bool act = (int)threadIdx.x < nthr;
+    C v[2][8];
+    if (act) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int r = 0; r < 8; ++r) v[c][(r & 1) * 4 + (r >> 1)] = buf[threadIdx.x + c * nthr + r * nb];  // slot 4 b + a
+    }
+    __syncthreads();
+    if (act) {
+        const int tstep = M / (Ns * 8);
+        const int lq = __ffs(M) - 3;  // log2(M / 4)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            C *u = v[c];
+            const int j = threadIdx.x + c * nthr;
+            const int k = j & (Ns - 1), t1 = k * tstep;
+            if (Ns > 1) {
+#pragma unroll
+                for (int a = 1; a < 4; ++a) {
+                    C w = tw_quarter<T>(stw, 2 * a * t1, lq);
+                    if (dir > 0) w.y = -w.y;
+                    u[a] = cmul(u[a], w);
+                    u[4 + a] = cmul(u[4 + a], w);
+                }
+            }
+            dft4(u[0], u[1], u[2], u[3], dir);
+            dft4(u[4], u[5], u[6], u[7], dir);
+            asm volatile("" ::: "memory");
+            const int idxD = (j - k) * 8 + k;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (q > 0 || Ns > 1) {
+                    C w = tw_quarter<T>(stw, t1 + q * (M >> 3), lq);
+                    if (dir > 0) w.y = -w.y;
+                    u[4 + q] = cmul(u[4 + q], w);
+                }
+                dft2(u[q], u[4 + q]);
+                buf[idxD + q * Ns] = u[q];
+                buf[idxD + (q + 4) * Ns] = u[4 + q];
+            }
             asm volatile("" ::: "memory");
         }
     }
@@ -239,6 +301,10 @@ __device__ __forceinline__ void fft_smem_e(cplx<T> *buf, int N, int dir, const c
             fft_pass16<T>(buf, N, Ns, dir, stw, M, nthr);
             Ns <<= 4;
             rem -= 4;
+        }
+        if (rem == 3) {
+            fft_pass8<T>(buf, N, Ns, dir, stw, M, nthr);
+            return;
         }
     }
     while (rem > 0) {
@@ -314,6 +380,27 @@ __device__ __forceinline__ cplx<T> *load_twiddles(cplx<T> *buf, int M, const cpl
     for (int u = threadIdx.x; u <= M / 4; u += blockDim.x) S[tw_swz<T>(u)] = tw[u * st];
     return S;
 }
+
+// us(i, ld(i)) for the block's i < n, B loads of a thread in flight: a block
+// fills an SM, so nothing else hides the latency of its global loads
+template <typename V, int B = 4, typename LD, typename US> __device__ __forceinline__ void batched(int n, LD ld, US us) {
+    for (int i0 = threadIdx.x; i0 < n; i0 += B * blockDim.x) {
+        V v[B];
+#pragma unroll
+        for (int c = 0; c < B; ++c) {
+            const int i = i0 + c * blockDim.x;
+            if (i < n) v[c] = ld(i);
+        }
+#pragma unroll
+        for (int c = 0; c < B; ++c) {
+            const int i = i0 + c * blockDim.x;
+            if (i < n) us(i, v[c]);
+        }
+    }
+}
+template <typename V> struct two_of {
+    V a, b;
+};
 
 template <typename T> __device__ __forceinline__ cplx<T> czero() { return mk<T>(cvt<T>(0.0), cvt<T>(0.0)); }
 
@@ -424,10 +511,13 @@ __global__ void __launch_bounds__(FFT_TPB)
     const double2 *col1 = H + (long long)c1 * ldH, *col2 = H + (long long)c2 * ldH;
     const int half = Nt / 2;
     const double dm1 = Dph[m1 + L], dm2 = two ? Dph[m1 + 1 + L] : 0.0;
-    for (int k = threadIdx.x; k < Nt; k += blockDim.x) {
+    auto ld_cols = [&](int k) {
+        const int kk = k <= half ? k : Nt - k;
+        return two_of<double2>{col1[kk], two ? col2[kk] : make_double2(0.0, 0.0)};
+    };
+    batched<two_of<double2>>(Nt, ld_cols, [&](int k, const two_of<double2> &cv) {
         const bool lo = k <= half;
-        const int kk = lo ? k : Nt - k;
-        double2 v1 = col1[kk], v2 = two ? col2[kk] : make_double2(0.0, 0.0);
+        double2 v1 = cv.a, v2 = cv.b;
         if constexpr (std::is_same<T, dfl>::value) {
             // split first, combine in double-float: no FP64 arithmetic (s2 = -s1)
             dfl ax = df_from(v1.x), ay = df_from(v1.y), bx = df_from(v2.x), by = df_from(v2.y);
@@ -443,26 +533,26 @@ __global__ void __launch_bounds__(FFT_TPB)
             }
             buf[k] = mk<T>(cvt<T>(v1.x - v2.y), cvt<T>(v1.y + v2.x));  // x1 + i x2
         }
-    }
+    });
     __syncthreads();
     fft_smem<T>(buf, Nt, -1, stw, Ntf);
     // separate, deconvolve, recombine; thread j owns the frequencies +-j
     // (reads j and Nt - j, writes j and Ntf - j: no other thread touches them);
     // the Nyquist term is dropped (Dth[half] = 0)
     const T hf = cvt<T>(0.5), ts1 = cvt<T>(s1), ts2 = cvt<T>(s2);
-    for (int j = threadIdx.x; j < half; j += blockDim.x) {
+    batched<double>(half, [&](int j) { return Dth[j]; }, [&](int j, double dt) {
         const int jn = j ? Nt - j : 0;
         const C zp = buf[j], zn = cscale(buf[jn], ts1);
         const C x1 = cscale(cadd(zp, zn), hf);
         const C d = cscale(csub(zp, zn), hf);
         const C x2 = mk<T>(d.y, -d.x);  // d / i
-        const C y1 = cscale(x1, scale_of<T>(Dth[j], dm1)), y2 = cscale(x2, scale_of<T>(Dth[j], dm2));
+        const C y1 = cscale(x1, scale_of<T>(dt, dm1)), y2 = cscale(x2, scale_of<T>(dt, dm2));
         buf[j] = mk<T>(y1.x - y2.y, y1.y + y2.x);  // y1 + i y2
         if (j) {
             const C y1n = cscale(y1, ts1), y2n = cscale(y2, ts2);  // Y_{-j} = s Y_j (D even)
             buf[Ntf - j] = mk<T>(y1n.x - y2n.y, y1n.y + y2n.x);
         }
-    }
+    });
     __syncthreads();
     // the inverse's input is zero in [half, Ntf - half] (Ntf / 4 = half): its
     // first radix-4 pass reads only x[j] and x[j + 3 Ntf / 4] (zero for j = 0),
@@ -586,19 +676,17 @@ __global__ void __launch_bounds__(FFT_TPB)
         // at m = Nb / 4 - j (m <= L); x[0] = (Re a_0, Re b_0)
         const cplx<T> *f1 = F + (long long)r1 * ncols, *f2 = F + (long long)r2 * ncols;
         const int nb = Nb / 4;
-        for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-            cplx<T> v0 = czero<T>(), v3 = czero<T>();
-            if (j < ncols) {
-                const cplx<T> a = f1[j], b = has2 ? f2[j] : czero<T>();
-                v0 = j ? mk<T>(a.x - b.y, a.y + b.x) : mk<T>(a.x, b.x);
-            }
-            const int m = nb - j;
-            if (m < ncols) {
-                const cplx<T> a = f1[m], b = has2 ? f2[m] : czero<T>();
-                v3 = mk<T>(a.x + b.y, b.x - a.y);
-            }
-            r4_first_pruned<T>(buf, j, v0, v3, +1);
-        }
+        auto ld_modes = [&](int j) {
+            two_of<two_of<cplx<T>>> v{{czero<T>(), czero<T>()}, {czero<T>(), czero<T>()}};
+            if (j < ncols) v.a.a = f1[j], v.a.b = has2 ? f2[j] : czero<T>();
+            if (nb - j < ncols) v.b.a = f1[nb - j], v.b.b = has2 ? f2[nb - j] : czero<T>();
+            return v;
+        };
+        batched<two_of<two_of<cplx<T>>>, 2>(nb, ld_modes, [&](int j, const two_of<two_of<cplx<T>>> &v) {
+            const cplx<T> a0 = v.a.a, b0 = v.a.b, a3 = v.b.a, b3 = v.b.b;
+            const cplx<T> v0 = j ? mk<T>(a0.x - b0.y, a0.y + b0.x) : mk<T>(a0.x, b0.x);
+            r4_first_pruned<T>(buf, j, v0, mk<T>(a3.x + b3.y, b3.x - a3.y), +1);
+        });
         __syncthreads();
         fft_smem<T>(buf, Nb, +1, stw, MTW, 2);
         TU *u1 = U + (long long)r1 * Npf;
@@ -658,10 +746,9 @@ __global__ void __launch_bounds__(FFT_TPB)
     const TU *u2 = U + (long long)r2 * Npf;
     const int Nb = Npf / SP;
     const int tstep = TW / Npf;
-    for (int j = threadIdx.x; j < Nb; j += blockDim.x) {
-        const int p = SP * j + q;
-        buf[j] = mk<T>(cvt<T>(to_d(u1[p])), cvt<T>(has2 ? to_d(u2[p]) : 0.0));
-    }
+    batched<two_of<TU>>(
+        Nb, [&](int j) { return two_of<TU>{u1[SP * j + q], has2 ? u2[SP * j + q] : TU(0)}; },
+        [&](int j, const two_of<TU> &u) { buf[j] = mk<T>(cvt<T>(to_d(u.a)), cvt<T>(to_d(u.b))); });
     __syncthreads();
     fft_smem<T>(buf, Nb, -1, stw, MTW);
     for (int m = threadIdx.x; m < ncols; m += blockDim.x) {
@@ -705,12 +792,11 @@ __global__ void __launch_bounds__(FFT_TPB)
     if constexpr (PRUNE) {
         const cplx<T> *row = F + (long long)r * ncols + L;  // mode m at row[m]
         const int nb = Nb / 4;
-        for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-            const cplx<T> v0 = j <= L ? row[j] : czero<T>();
-            const int m3 = j - nb;  // the mode at x[j + 3 Nb / 4]
-            const cplx<T> v3 = m3 >= -L ? row[m3] : czero<T>();
-            r4_first_pruned<T>(buf, j, v0, v3, +1);
-        }
+        auto ld_modes = [&](int j) {  // j - nb: the mode at x[j + 3 Nb / 4]
+            return two_of<cplx<T>>{j <= L ? row[j] : czero<T>(), j - nb >= -L ? row[j - nb] : czero<T>()};
+        };
+        batched<two_of<cplx<T>>>(
+            nb, ld_modes, [&](int j, const two_of<cplx<T>> &v) { r4_first_pruned<T>(buf, j, v.a, v.b, +1); });
         __syncthreads();
         fft_smem<T>(buf, Nb, +1, stw, MTW, 2);
         for (int j = threadIdx.x; j < Nb; j += blockDim.x) U[(long long)r * Npf + j] = ccast<TU>(buf[j]);
@@ -742,10 +828,9 @@ __global__ void __launch_bounds__(FFT_TPB)
     const int ncols = 2 * L + 1;
     const int Nb = Npf / SP;
     const int tstep = TW / Npf;
-    for (int j = threadIdx.x; j < Nb; j += blockDim.x) {
-        const cplx<TU> u = U[(long long)r * Npf + SP * j + q];
-        buf[j] = mk<T>(cvt<T>(to_d(u.x)), cvt<T>(to_d(u.y)));
-    }
+    batched<cplx<TU>>(
+        Nb, [&](int j) { return U[(long long)r * Npf + SP * j + q]; },
+        [&](int j, const cplx<TU> &u) { buf[j] = mk<T>(cvt<T>(to_d(u.x)), cvt<T>(to_d(u.y))); });
     __syncthreads();
     fft_smem<T>(buf, Nb, -1, stw, MTW);
     for (int c = threadIdx.x; c < ncols; c += blockDim.x) {
@@ -1047,34 +1132,38 @@ __global__ void __launch_bounds__(FFT_TPB)
         const int r = wrap2(n - n_lo, Ntf);
         return r < nrows ? F[(long long)r * ncols + c] : czero<T>();
     };
-    for (int n = threadIdx.x; n <= Ntf / 2; n += blockDim.x) {
+    auto ld_rows = [&](int n) {
         const int nn = wrap2(-n, Ntf);
-        const C a1 = row(n, c1), b1 = row(nn, c1);
-        const C a2 = two ? row(n, c2) : czero<T>(), b2 = two ? row(nn, c2) : czero<T>();
+        return two_of<two_of<C>>{{row(n, c1), two ? row(n, c2) : czero<T>()},
+                                 {row(nn, c1), two ? row(nn, c2) : czero<T>()}};
+    };
+    batched<two_of<two_of<C>>, 2>(Ntf / 2 + 1, ld_rows, [&](int n, const two_of<two_of<C>> &v) {
+        const int nn = wrap2(-n, Ntf);
+        const C a1 = v.a.a, b1 = v.b.a, a2 = v.a.b, b2 = v.b.b;
         const C p1 = cscale(cadd(a1, cscale(b1, ts1)), hf), p2 = cscale(cadd(a2, cscale(b2, ts2)), hf);
         buf[n] = mk<T>(p1.x - p2.y, p1.y + p2.x);
         if (nn != n) {
             const C q1 = cscale(p1, ts1), q2 = cscale(p2, ts2);
             buf[nn] = mk<T>(q1.x - q2.y, q1.y + q2.x);
         }
-    }
+    });
     __syncthreads();
     fft_smem<T>(buf, Ntf, -1, stw, Ntf);
     // separate, deconvolve, recombine into the Nt-point band; thread j owns +-j
     // (reads j and Ntf - j, writes j and Nt - j); the Nyquist term is zero
-    for (int j = threadIdx.x; j < half; j += blockDim.x) {
+    batched<double>(half, [&](int j) { return Dth[j]; }, [&](int j, double dt) {
         const int jn = j ? Ntf - j : 0;
         const C zp = buf[j], zn = cscale(buf[jn], ts1);
         const C x1 = cscale(cadd(zp, zn), hf);
         const C d = cscale(csub(zp, zn), hf);
         const C x2 = mk<T>(d.y, -d.x);
-        const C y1 = cscale(x1, scale_of<T>(Dth[j], dm1)), y2 = cscale(x2, scale_of<T>(Dth[j], dm2));
+        const C y1 = cscale(x1, scale_of<T>(dt, dm1)), y2 = cscale(x2, scale_of<T>(dt, dm2));
         buf[j] = mk<T>(y1.x - y2.y, y1.y + y2.x);
         if (j) {
             const C y1n = cscale(y1, ts1), y2n = cscale(y2, ts2);
             buf[Nt - j] = mk<T>(y1n.x - y2n.y, y1n.y + y2n.x);
         }
-    }
+    });
     if (threadIdx.x == 0) buf[half] = czero<T>();
     __syncthreads();
     fft_smem<T>(buf, Nt, +1, stw, Ntf);
