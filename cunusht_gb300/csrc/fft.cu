@@ -123,7 +123,14 @@ __device__ __forceinline__ cplx<T> tw_quarter(const cplx<T> *S, int t, int lq) {
     return mk<T>(x, y);
 }
 
-template <typename T, int R, int NB>
+// Product with a twiddle. FP32: fixed fused operations, the ones the compiler
+// makes of cmul in fft_pass_e, so that passes joined in registers round alike.
+template <typename C> __device__ __forceinline__ C tw_mul(C a, C b) { return cmul(a, b); }
+__device__ __forceinline__ float2 tw_mul(float2 a, float2 b) {
+    return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+
+template <typename T, int R, int NB, bool SMALL = false>
 __device__ __forceinline__ void fft_pass_e(cplx<T> *buf, int N, int Ns, int dir,
                                            const cplx<T> *__restrict__ stw, int M, int nthr) {
     using C = cplx<T>;
@@ -151,7 +158,7 @@ __device__ __forceinline__ void fft_pass_e(cplx<T> *buf, int N, int Ns, int dir,
                 for (int r = 1; r < R; ++r) {
                     C w = tw_quarter<T>(stw, r * k * tstep, lq);
                     if (dir > 0) w.y = -w.y;
-                    v[c][r] = cmul(v[c][r], w);
+                    v[c][r] = SMALL ? tw_mul(v[c][r], w) : cmul(v[c][r], w);
                 }
             }
             dftR<T, R>(v[c], dir);
@@ -166,8 +173,8 @@ __device__ __forceinline__ void fft_pass_e(cplx<T> *buf, int N, int Ns, int dir,
     __syncthreads();
 }
 
-// One radix-16 pass of the FP64 and double-float transforms with 16 elements
-// per thread: two radix-4 stages in registers, so it costs the shared-memory
+// One radix-16 pass with 16 elements
+// per thread (FP64 and double-float transforms, FP32 ones of 2048 points): two radix-4 stages in registers, so it costs the shared-memory
 // round trip and the two barriers of one pass for the work of two.  Element
 // r = 4 a + b of the butterfly: radix-4 over a with the twiddles w^(4 a k), the
 // factors e^{dir 2 pi i b q / 16} w^(b k), radix-4 over b.  In place in v, whose
@@ -202,7 +209,7 @@ __device__ __forceinline__ void fft_pass16(cplx<T> *buf, int N, int Ns, int dir,
             C *u = v + 4 * b;
             if (Ns > 1) {
 #pragma unroll
-                for (int a = 1; a < 4; ++a) u[a] = cmul(u[a], w4[a - 1]);
+                for (int a = 1; a < 4; ++a) u[a] = tw_mul(u[a], w4[a - 1]);
             }
             dft4(u[0], u[1], u[2], u[3], dir);  // u[q]: frequency q over a
             asm volatile("" ::: "memory");
@@ -215,7 +222,7 @@ __device__ __forceinline__ void fft_pass16(cplx<T> *buf, int N, int Ns, int dir,
                 // w^(b k) e^{-2 pi i b q / 16}: table index b (t1 + q M / 16)
                 C w = tw_quarter<T>(stw, b * (t1 + q * (M >> 4)), lq);
                 if (dir > 0) w.y = -w.y;
-                v[4 * b + q] = cmul(v[4 * b + q], w);
+                v[4 * b + q] = tw_mul(v[4 * b + q], w);
             }
             dft4(v[q], v[4 + q], v[8 + q], v[12 + q], dir);
             const int idxD = (j - k) * 16 + k;
@@ -259,8 +266,8 @@ __device__ __forceinline__ void fft_pass8(cplx<T> *buf, int N, int Ns, int dir, 
                 for (int a = 1; a < 4; ++a) {
                     C w = tw_quarter<T>(stw, 2 * a * t1, lq);
                     if (dir > 0) w.y = -w.y;
-                    u[a] = cmul(u[a], w);
-                    u[4 + a] = cmul(u[4 + a], w);
+                    u[a] = tw_mul(u[a], w);
+                    u[4 + a] = tw_mul(u[4 + a], w);
                 }
             }
             dft4(u[0], u[1], u[2], u[3], dir);
@@ -272,7 +279,7 @@ __device__ __forceinline__ void fft_pass8(cplx<T> *buf, int N, int Ns, int dir, 
                 if (q > 0 || Ns > 1) {
                     C w = tw_quarter<T>(stw, t1 + q * (M >> 3), lq);
                     if (dir > 0) w.y = -w.y;
-                    u[4 + q] = cmul(u[4 + q], w);
+                    u[4 + q] = tw_mul(u[4 + q], w);
                 }
                 dft2(u[q], u[4 + q]);
                 buf[idxD + q * Ns] = u[q];
@@ -323,6 +330,88 @@ __device__ __forceinline__ void fft_smem_e(cplx<T> *buf, int N, int dir, const c
     }
 }
 
+// S radix-2 passes of a transform in one round trip (FFT_SMALL_TPB threads, one
+// group of 2^S elements each).  With q the output bits of the stages done, stage s
+// takes the pairs r, r + R / 2^(s+1) with the twiddle w^(k + q Ns) of a pass of
+// 2^(s+1) Ns points: the operations of the single passes.
+template <typename T, int S>
+__device__ __forceinline__ void fft_pass2s(cplx<T> *buf, int N, int Ns, int dir, const cplx<T> *__restrict__ stw,
+                                           int M) {
+    using C = cplx<T>;
+    constexpr int R = 1 << S;
+    const int nb = N / R;  // <= blockDim
+    const bool act = (int)threadIdx.x < nb;
+    const int j = threadIdx.x;
+    C v[R];
+    if (act) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = buf[j + r * nb];
+    }
+    __syncthreads();
+    if (act) {
+        const int lq = __ffs(M) - 3;  // log2(M / 4)
+        const int k = j & (Ns - 1);
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const int tstep = M / ((2 << s) * Ns), h = R >> (s + 1);
+            C u[R];
+#pragma unroll
+            for (int q = 0; q < (1 << s); ++q) {
+                C w = mk<T>(cvt<T>(1.0), cvt<T>(0.0));
+                if (s > 0 || Ns > 1) {
+                    w = tw_quarter<T>(stw, (k + q * Ns) * tstep, lq);
+                    if (dir > 0) w.y = -w.y;
+                }
+#pragma unroll
+                for (int r = 0; r < h; ++r) {
+                    C a = v[q * 2 * h + r], b = v[q * 2 * h + h + r];
+                    if (s > 0 || Ns > 1) b = tw_mul(b, w);
+                    dft2(a, b);
+                    u[q * h + r] = a;
+                    u[(q + (1 << s)) * h + r] = b;
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = u[r];
+        }
+        const int idxD = (j - k) * R + k;
+#pragma unroll
+        for (int q = 0; q < R; ++q) buf[idxD + q * Ns] = v[q];
+    }
+    __syncthreads();
+}
+
+// the one or two radix-2 passes left of up to 1024 points
+template <typename T>
+__device__ __forceinline__ void fft_tail2(cplx<T> *buf, int N, int Ns, int dir, const cplx<T> *__restrict__ stw, int M,
+                                          int rem) {
+    for (; rem > 0; --rem, Ns <<= 1) {
+        if (N > 4 * FFT_SMALL_TPB) fft_pass_e<T, 2, 4, true>(buf, N, Ns, dir, stw, M, N / 8);
+        else fft_pass_e<T, 2, 2, true>(buf, N, Ns, dir, stw, M, N / 4);
+    }
+}
+
+// Transforms of up to 2048 points in a block of FFT_SMALL_TPB threads: the
+// passes that FFT_TPB threads take (radix 4 above 1024 points, radix 2 up to
+// there), two to four of them per round trip, so that a transform's result
+// doesn't depend on the block's size.
+template <typename T>
+__device__ __forceinline__ void fft_smem_small(cplx<T> *buf, int N, int dir, const cplx<T> *__restrict__ stw, int M,
+                                               int l0) {
+    int rem = __ffs(N) - 1 - l0;
+    int Ns = 1 << l0;
+    if (N > 2 * FFT_TPB) {
+        constexpr int nthr = FFT_SMALL_TPB;
+        for (; rem >= 4; rem -= 4, Ns <<= 4) fft_pass16<T>(buf, N, Ns, dir, stw, M, nthr);
+        if (rem == 3) fft_pass8<T>(buf, N, Ns, dir, stw, M, nthr);
+        else if (rem == 2) fft_pass_e<T, 4, 4, true>(buf, N, Ns, dir, stw, M, nthr);
+        else if (rem == 1) fft_pass_e<T, 2, 8, true>(buf, N, Ns, dir, stw, M, nthr);
+        return;
+    }
+    for (; rem >= 3; rem -= 3, Ns <<= 3) fft_pass2s<T, 3>(buf, N, Ns, dir, stw, M);
+    if (rem > 0) fft_tail2<T>(buf, N, Ns, dir, stw, M, rem);
+}
+
 // In-place FFT of length N (power of two, 2 <= N <= 16 blockDim) in shared
 // memory.  dir = -1: X_k = sum_n x_n e^{-2 pi i nk/N}; dir = +1: the
 // unnormalised inverse.  stw: the quarter twiddle table of length M >= N in
@@ -332,7 +421,9 @@ template <typename T>
 __device__ __forceinline__ void fft_smem(cplx<T> *buf, int N, int dir, const cplx<T> *__restrict__ stw, int M,
                                          int l0 = 0) {
     const int B = blockDim.x;
-    if (N > 8 * B) {
+    if (B == FFT_SMALL_TPB) {
+        fft_smem_small<T>(buf, N, dir, stw, M, l0);
+    } else if (N > 8 * B) {
         // 16 elements per thread: radix <= 8 for float, <= 4 for double and
         // double-float keeps the pass within the 128-register budget of a
         // 512-thread block
@@ -1032,6 +1123,16 @@ __global__ void __launch_bounds__(FFT_TPB)
 }
 
 // ------------------------------------------------------------ host launchers
+// Threads of a transform block of N points.  A block of FFT_TPB threads fills
+// an SM with its registers, and at 4 points a thread or fewer it waits on
+// barriers and loads: four blocks of FFT_SMALL_TPB threads cover each other's,
+// and their passes hold more points (eight spin-2 requests at lmax 511, FP32:
+// theta 0.307 -> 0.143 ms, phi 0.246 -> 0.094).  Launches that leave SMs idle keep the large
+// blocks.
+static int fft_threads(int N, long long blocks) {
+    return N <= 16 * FFT_SMALL_TPB && N >= 4 * FFT_SMALL_TPB && blocks >= 4 * 152 ? FFT_SMALL_TPB : FFT_TPB;
+}
+
 template <typename K> static int set_smem(K kernel, size_t bytes) {
     if (bytes > 48 * 1024) CU_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     return CUNUSHT_OK;
@@ -1054,19 +1155,20 @@ int theta_fwd_batch(const cunusht_plan_s *P, int nreq, int spin, const double2 *
     dim3 grid(ncols, nreq, P->sp_theta);
     if (P->sp_theta == 1) {  // two columns per block
         const dim3 g2((ncols + 1) / 2, nreq);
+        const int tpb = fft_threads(P->Ntf, (long long)g2.x * nreq);
         if (P->grid_fp32) {
             RC_TRY(set_smem(k_theta_fwd2<float>, sm));
-            k_theta_fwd2<float><<<g2, FFT_TPB, sm, st>>>(H, P->ncc, P->Nt, P->Ntf, spin, mofs, L, P->d_Dth, P->d_Dph,
+            k_theta_fwd2<float><<<g2, tpb, sm, st>>>(H, P->ncc, P->Nt, P->Ntf, spin, mofs, L, P->d_Dth, P->d_Dph,
                                                          (float2 *)F, ncols, P->n_lo, P->nrows, P->d_tw32, P->TW, hbs,
                                                          fbs);
         } else if (P->fft_df) {
             RC_TRY(set_smem(k_theta_fwd2<dfl>, sm));
-            k_theta_fwd2<dfl><<<g2, FFT_TPB, sm, st>>>(H, P->ncc, P->Nt, P->Ntf, spin, mofs, L, P->d_Dth, P->d_Dph,
+            k_theta_fwd2<dfl><<<g2, tpb, sm, st>>>(H, P->ncc, P->Nt, P->Ntf, spin, mofs, L, P->d_Dth, P->d_Dph,
                                                        (dcplx *)F, ncols, P->n_lo, P->nrows, (const dcplx *)P->d_twdf,
                                                        P->TW, hbs, fbs);
         } else {
             RC_TRY(set_smem(k_theta_fwd2<double>, sm));
-            k_theta_fwd2<double><<<g2, FFT_TPB, sm, st>>>(H, P->ncc, P->Nt, P->Ntf, spin, mofs, L, P->d_Dth,
+            k_theta_fwd2<double><<<g2, tpb, sm, st>>>(H, P->ncc, P->Nt, P->Ntf, spin, mofs, L, P->d_Dth,
                                                           P->d_Dph, (double2 *)F, ncols, P->n_lo, P->nrows,
                                                           P->d_tw64, P->TW, hbs, fbs);
         }
@@ -1191,19 +1293,20 @@ int theta_adj_batch(const cunusht_plan_s *P, int nreq, int spin, const void *F, 
     dim3 grid(ncols, nreq);
     if (SP == 1) {  // two columns per block
         const dim3 g2((ncols + 1) / 2, nreq);
+        const int tpb = fft_threads(P->Ntf, (long long)g2.x * nreq);
         if (P->grid_fp32) {
             RC_TRY(set_smem(k_theta_adj2<float>, sm));
-            k_theta_adj2<float><<<g2, FFT_TPB, sm, st>>>((const float2 *)F, ncols, P->n_lo, P->nrows, P->Nt, P->Ntf,
+            k_theta_adj2<float><<<g2, tpb, sm, st>>>((const float2 *)F, ncols, P->n_lo, P->nrows, P->Nt, P->Ntf,
                                                          spin, mofs, L, P->d_Dth, P->d_Dph, H, P->ncc, P->d_tw32,
                                                          P->TW, fbs, hbs);
         } else if (P->fft_df) {
             RC_TRY(set_smem(k_theta_adj2<dfl>, sm));
-            k_theta_adj2<dfl><<<g2, FFT_TPB, sm, st>>>((const dcplx *)F, ncols, P->n_lo, P->nrows, P->Nt, P->Ntf,
+            k_theta_adj2<dfl><<<g2, tpb, sm, st>>>((const dcplx *)F, ncols, P->n_lo, P->nrows, P->Nt, P->Ntf,
                                                        spin, mofs, L, P->d_Dth, P->d_Dph, H, P->ncc,
                                                        (const dcplx *)P->d_twdf, P->TW, fbs, hbs);
         } else {
             RC_TRY(set_smem(k_theta_adj2<double>, sm));
-            k_theta_adj2<double><<<g2, FFT_TPB, sm, st>>>((const double2 *)F, ncols, P->n_lo, P->nrows, P->Nt,
+            k_theta_adj2<double><<<g2, tpb, sm, st>>>((const double2 *)F, ncols, P->n_lo, P->nrows, P->Nt,
                                                           P->Ntf, spin, mofs, L, P->d_Dth, P->d_Dph, H, P->ncc,
                                                           P->d_tw64, P->TW, fbs, hbs);
         }
@@ -1246,13 +1349,14 @@ static int phi_fwd_s0_launch(const cunusht_plan_s *P, int nreq, const void *F, l
                              const cplx<T> *tw, size_t sm, cudaStream_t st) {
     const int L = P->lmax, SP = P->sp_phi;
     const dim3 grid((P->nrows + 1) / 2, nreq, SP);
+    const int tpb = fft_threads(P->Npf / SP, (long long)grid.x * nreq * SP);
     if (SP == 1 && P->Npf / 4 > L) {
         RC_TRY(set_smem(k_phi_fwd_s0<T, TU, true>, sm));
-        k_phi_fwd_s0<T, TU, true><<<grid, FFT_TPB, sm, st>>>((const cplx<T> *)F, L + 1, P->nrows, P->Npf, (TU *)U, tw,
+        k_phi_fwd_s0<T, TU, true><<<grid, tpb, sm, st>>>((const cplx<T> *)F, L + 1, P->nrows, P->Npf, (TU *)U, tw,
                                                               P->TW, fbs, ubs, SP);
     } else {
         RC_TRY(set_smem(k_phi_fwd_s0<T, TU, false>, sm));
-        k_phi_fwd_s0<T, TU, false><<<grid, FFT_TPB, sm, st>>>((const cplx<T> *)F, L + 1, P->nrows, P->Npf, (TU *)U,
+        k_phi_fwd_s0<T, TU, false><<<grid, tpb, sm, st>>>((const cplx<T> *)F, L + 1, P->nrows, P->Npf, (TU *)U,
                                                                tw, P->TW, fbs, ubs, SP);
     }
     return CUNUSHT_OK;
@@ -1265,13 +1369,14 @@ static int phi_fwd_spin_launch(const cunusht_plan_s *P, int nreq, const void *F,
                                const cplx<T> *tw, size_t sm, cudaStream_t st) {
     const int L = P->lmax, SP = P->sp_phi;
     const dim3 grid(P->nrows, nreq, SP);
+    const int tpb = fft_threads(P->Npf / SP, (long long)grid.x * nreq * SP);
     if (SP == 1 && P->Npf / 4 > L) {
         RC_TRY(set_smem(k_phi_fwd_spin<T, TU, true>, sm));
-        k_phi_fwd_spin<T, TU, true><<<grid, FFT_TPB, sm, st>>>((const cplx<T> *)F, L, P->Npf, (cplx<TU> *)U, tw,
+        k_phi_fwd_spin<T, TU, true><<<grid, tpb, sm, st>>>((const cplx<T> *)F, L, P->Npf, (cplx<TU> *)U, tw,
                                                                 P->TW, fbs, ubs, SP);
     } else {
         RC_TRY(set_smem(k_phi_fwd_spin<T, TU, false>, sm));
-        k_phi_fwd_spin<T, TU, false><<<grid, FFT_TPB, sm, st>>>((const cplx<T> *)F, L, P->Npf, (cplx<TU> *)U, tw,
+        k_phi_fwd_spin<T, TU, false><<<grid, tpb, sm, st>>>((const cplx<T> *)F, L, P->Npf, (cplx<TU> *)U, tw,
                                                                  P->TW, fbs, ubs, SP);
     }
     return CUNUSHT_OK;
@@ -1320,34 +1425,36 @@ int phi_adj_batch(const cunusht_plan_s *P, int nreq, int spin, const void *U, lo
     for (int q = SP - 1; q >= 0; --q) {
         if (spin == 0) {
             const dim3 grid((P->nrows + 1) / 2, nreq);
+            const int tpb = fft_threads(P->Npf / SP, (long long)grid.x * nreq);
             if (P->grid_fp32) {
                 RC_TRY(set_smem(k_phi_adj_s0<float>, sm));
-                k_phi_adj_s0<float><<<grid, FFT_TPB, sm, st>>>((const float *)U, P->nrows, P->Npf, (float2 *)F, L + 1,
+                k_phi_adj_s0<float><<<grid, tpb, sm, st>>>((const float *)U, P->nrows, P->Npf, (float2 *)F, L + 1,
                                                                P->d_tw32, P->TW, SP, q, ubs, fbs);
             } else if (P->fft_df) {  // FP64 grid, double-float transforms
                 RC_TRY(set_smem(k_phi_adj_s0<dfl, double>, sm));
-                k_phi_adj_s0<dfl, double><<<grid, FFT_TPB, sm, st>>>((const double *)U, P->nrows, P->Npf, (dcplx *)F,
+                k_phi_adj_s0<dfl, double><<<grid, tpb, sm, st>>>((const double *)U, P->nrows, P->Npf, (dcplx *)F,
                                                                      L + 1, (const dcplx *)P->d_twdf, P->TW, SP, q,
                                                                      ubs, fbs);
             } else {
                 RC_TRY(set_smem(k_phi_adj_s0<double>, sm));
-                k_phi_adj_s0<double><<<grid, FFT_TPB, sm, st>>>((const double *)U, P->nrows, P->Npf, (double2 *)F,
+                k_phi_adj_s0<double><<<grid, tpb, sm, st>>>((const double *)U, P->nrows, P->Npf, (double2 *)F,
                                                                 L + 1, P->d_tw64, P->TW, SP, q, ubs, fbs);
             }
         } else {
             const dim3 grid(P->nrows, nreq);
+            const int tpb = fft_threads(P->Npf / SP, (long long)grid.x * nreq);
             if (P->grid_fp32) {
                 RC_TRY(set_smem(k_phi_adj_spin<float>, sm));
-                k_phi_adj_spin<float><<<grid, FFT_TPB, sm, st>>>((const float2 *)U, L, P->Npf, (float2 *)F,
+                k_phi_adj_spin<float><<<grid, tpb, sm, st>>>((const float2 *)U, L, P->Npf, (float2 *)F,
                                                                  P->d_tw32, P->TW, SP, q, ubs / 2, fbs);
             } else if (P->fft_df) {
                 RC_TRY(set_smem(k_phi_adj_spin<dfl, double>, sm));
-                k_phi_adj_spin<dfl, double><<<grid, FFT_TPB, sm, st>>>((const double2 *)U, L, P->Npf, (dcplx *)F,
+                k_phi_adj_spin<dfl, double><<<grid, tpb, sm, st>>>((const double2 *)U, L, P->Npf, (dcplx *)F,
                                                                        (const dcplx *)P->d_twdf, P->TW, SP, q,
                                                                        ubs / 2, fbs);
             } else {
                 RC_TRY(set_smem(k_phi_adj_spin<double>, sm));
-                k_phi_adj_spin<double><<<grid, FFT_TPB, sm, st>>>((const double2 *)U, L, P->Npf, (double2 *)F,
+                k_phi_adj_spin<double><<<grid, tpb, sm, st>>>((const double2 *)U, L, P->Npf, (double2 *)F,
                                                                   P->d_tw64, P->TW, SP, q, ubs / 2, fbs);
             }
         }

@@ -5,6 +5,7 @@
 namespace cunusht {
 
 constexpr int FFT_TPB = 512;
+constexpr int FFT_SMALL_TPB = 128;  // of transforms up to 2048 points, where the launch fills the GPU
 
 // capi.cu: device allocation counted in the plan's workspace bytes
 int plan_alloc(cunusht_plan_s *P, void **p, size_t bytes);
