@@ -472,27 +472,6 @@ __device__ __forceinline__ cplx<T> *load_twiddles(cplx<T> *buf, int M, const cpl
     return S;
 }
 
-// us(i, ld(i)) for the block's i < n, B loads of a thread in flight: a block
-// fills an SM, so nothing else hides the latency of its global loads
-template <typename V, int B = 4, typename LD, typename US> __device__ __forceinline__ void batched(int n, LD ld, US us) {
-    for (int i0 = threadIdx.x; i0 < n; i0 += B * blockDim.x) {
-        V v[B];
-#pragma unroll
-        for (int c = 0; c < B; ++c) {
-            const int i = i0 + c * blockDim.x;
-            if (i < n) v[c] = ld(i);
-        }
-#pragma unroll
-        for (int c = 0; c < B; ++c) {
-            const int i = i0 + c * blockDim.x;
-            if (i < n) us(i, v[c]);
-        }
-    }
-}
-template <typename V> struct two_of {
-    V a, b;
-};
-
 template <typename T> __device__ __forceinline__ cplx<T> czero() { return mk<T>(cvt<T>(0.0), cvt<T>(0.0)); }
 
 // e^{dirsign 2 pi i k / TW'} from the table, tstep = TW / TW' (TW' | TW,
@@ -964,11 +943,13 @@ __device__ __forceinline__ void ring_class(const RingCls &rc, int ring, int &N, 
 
 // The FP64 sincos of m phi0 was a third of the ring transform of grids whose rings
 // start off zero (HEALPix): it is evaluated once for m and -m, into a table in
-// shared memory behind the twiddles, where the block has room for one (nside
-// 512, lmax 1000, double-float: 1.17 -> 0.79 ms; the same sines and cosines).
+// shared memory behind the twiddles (nside 512, lmax 1000, double-float: 1.17
+// -> 0.79 ms; the same sines and cosines), up to 200 KB in all: a table that
+// takes the last of the L1 cache made the 16384-point rings of lmax 4095 8 %
+// slower (4.9 -> 5.3 ms).
 __host__ __device__ inline size_t ring_phase_bytes(int L, size_t sm) {
     const size_t b = (size_t)(L + 1) * sizeof(double2);
-    return sm + b <= 227 * 1024 ? b : 0;
+    return sm + b <= 200 * 1024 ? b : 0;
 }
 
 template <typename T>

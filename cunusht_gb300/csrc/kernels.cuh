@@ -7,6 +7,27 @@ namespace cunusht {
 constexpr int FFT_TPB = 512;
 constexpr int FFT_SMALL_TPB = 128;  // of transforms up to 2048 points, where the launch fills the GPU
 
+// us(i, ld(i)) for the block's i < n, B loads of a thread in flight: a block
+// fills an SM, so nothing else hides the latency of its global loads
+template <typename V, int B = 4, typename LD, typename US> __device__ __forceinline__ void batched(int n, LD ld, US us) {
+    for (int i0 = threadIdx.x; i0 < n; i0 += B * blockDim.x) {
+        V v[B];
+#pragma unroll
+        for (int c = 0; c < B; ++c) {
+            const int i = i0 + c * blockDim.x;
+            if (i < n) v[c] = ld(i);
+        }
+#pragma unroll
+        for (int c = 0; c < B; ++c) {
+            const int i = i0 + c * blockDim.x;
+            if (i < n) us(i, v[c]);
+        }
+    }
+}
+template <typename V> struct two_of {
+    V a, b;
+};
+
 // capi.cu: device allocation counted in the plan's workspace bytes
 int plan_alloc(cunusht_plan_s *P, void **p, size_t bytes);
 

@@ -223,27 +223,39 @@ __global__ void __launch_bounds__(MR_TPB, 2)
     for (int i = 0; i < st.n; ++i)
         for (int m = threadIdx.x; m < st.R[i]; m += blockDim.x) K[st.coff[i] + m] = tw[m * (N / st.R[i])];
     const double ph0 = phi0[ring];
-    for (int qi = threadIdx.x; qi < N; qi += blockDim.x) {
-        // bin qi gathers every m = qi (mod N); with N >= 2L + 1 (no aliasing) one term.
-        // Double-float sums for the mixed path: no FP64 arithmetic unless phi0 != 0
-        T ax = cvt<T>(0.0), ay = cvt<T>(0.0);
-        for (int m = qi - N * ((qi + L) / N); m <= L; m += N) {
-            double2 h;
-            if (spin == 0) {
-                const double2 hm = Hgl[(long long)(m < 0 ? -m : m) * nring + ring];
-                h = m == 0 ? make_double2(hm.x, 0.0) : (m > 0 ? hm : make_double2(hm.x, -hm.y));
-            } else {
-                h = Hgl[(long long)(m + L) * nring + ring];
-            }
-            if (ph0 != 0.0 && m != 0) {
-                double sn, cs;
-                sincos(m * ph0, &sn, &cs);
-                h = cmul(h, make_double2(cs, sn));
-            }
-            ax = ax + cvt<T>(h.x);
-            ay = ay + cvt<T>(h.y);
+    // bin qi gathers every m = qi (mod N).  Double-float sums for the mixed path: no FP64
+    // arithmetic unless phi0 != 0
+    auto mode = [&](int m) -> double2 {
+        if (spin != 0) return Hgl[(long long)(m + L) * nring + ring];
+        const double2 hm = Hgl[(long long)(m < 0 ? -m : m) * nring + ring];
+        return m == 0 ? make_double2(hm.x, 0.0) : (m > 0 ? hm : make_double2(hm.x, -hm.y));
+    };
+    auto add = [&](T &ax, T &ay, int m, double2 h) {
+        if (ph0 != 0.0 && m != 0) {
+            double sn, cs;
+            sincos(m * ph0, &sn, &cs);
+            h = cmul(h, make_double2(cs, sn));
         }
-        buf[qi] = mk<T>(ax, ay);
+        ax = ax + cvt<T>(h.x);
+        ay = ay + cvt<T>(h.y);
+    };
+    if (N > 2 * L) {
+        // at most one term: the strided loads go out together (eight requests
+        // at lmax 2047: 3.12 -> 2.98 ms)
+        auto at = [&](int qi) { return qi <= L ? qi : qi - N; };
+        batched<double2>(
+            N, [&](int qi) { return at(qi) >= -L ? mode(at(qi)) : make_double2(0.0, 0.0); },
+            [&](int qi, const double2 &h) {
+                T ax = cvt<T>(0.0), ay = cvt<T>(0.0);
+                if (at(qi) >= -L) add(ax, ay, at(qi), h);
+                buf[qi] = mk<T>(ax, ay);
+            });
+    } else {
+        for (int qi = threadIdx.x; qi < N; qi += blockDim.x) {
+            T ax = cvt<T>(0.0), ay = cvt<T>(0.0);
+            for (int m = qi - N * ((qi + L) / N); m <= L; m += N) add(ax, ay, m, mode(m));
+            buf[qi] = mk<T>(ax, ay);
+        }
     }
     __syncthreads();
     mr_fft<T>(buf, N, st, K, tw);
