@@ -28,10 +28,16 @@
 // the products are more accurate than the double-float CUDA-core kernels,
 // which round every product to FP32.
 //
-// Block: one order m and 256 ring pairs as four 128-row MMA tiles (544
-// threads) for launches of up to 4 requests, 192 ring pairs as three tiles
-// (416 threads) for 8 requests, whose 160 tensor-memory columns per tile fit
-// 512 three times.  Each ring thread holds one ring (the first half of them the
+// The FMA pipe bounds it (about 70 % busy): the recursion and the digit split
+// run in packed FP32 for two l, which halves their issue slots, and with up to
+// 2 requests two blocks of two 128-row MMA tiles share an SM.  One request,
+// spin 2, lmax 4095: 50.8 -> 41.2 ms; spin 0, lmax 3087: 15.0 -> 10.5 ms;
+// eight requests at lmax 2047: 9.05 -> 8.26 ms.
+//
+// Block: one order m and 128 ring pairs as two 128-row MMA tiles for launches
+// of up to 2 requests, 256 ring pairs as four tiles (544 threads) for 4, 192 ring
+// pairs as three tiles (416 threads) for 8 requests, whose 160 tensor-memory
+// columns per tile fit 512 three times.  Each ring thread holds one ring (the first half of them the
 // rings theta, the second half pi - theta); per chunk of 16 l it writes its
 // four digit rows (two 16-byte K-cores per digit) into the A tile, and the
 // ring threads together write the B' digits.  The last warp issues tiles x 4

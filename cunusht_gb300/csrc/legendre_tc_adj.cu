@@ -35,7 +35,9 @@
 // 2^U(l, request) from a bound on |D|).  A finish kernel turns the sums into
 // alm (the same combinations as the double-float CUDA-core kernel,
 // legendre.cu k_leg_adj_*_df).  Every wait is bounded; on a timeout the block
-// sets bit 0 of the plan's status word and returns.
+// sets bit 0 of the plan's status word and returns.  The ring warps' FP32
+// arithmetic bounds it; two l at a time in packed FP32, four spin-2 requests at
+// lmax 2047: 12.7 -> 10.2 ms.
 #include "common.cuh"
 #include "df.cuh"
 #include "kernels.cuh"
