@@ -857,9 +857,10 @@ __global__ void __launch_bounds__(256)
     const double nz = ct * cosa - st * t * sinaoa;
     const double rho = sqrt(nx * nx + ny * ny);
     // the increments from their series where they are small (all but the pixels next to a pole):
-    // theta' - theta = asin(rho ct - nz st), phi' - phi = -atan(ny / nx)
-    const double sd = rho * ct - nz * st;
-    oth[j] = fabs(sd) < 0.02 ? theta + asin_small(sd) : atan2(rho, nz);
+    // theta' - theta = asin(rho ct - nz st), phi' - phi = -atan(ny / nx).  The sine is as small where
+    // a pixel next to one pole moves next to the other: there the cosine is negative
+    const double sd = rho * ct - nz * st, cd = rho * st + nz * ct;
+    oth[j] = fabs(sd) < 0.02 && cd > 0.0 ? theta + asin_small(sd) : atan2(rho, nz);
     const double q = ny / nx;
     double php = phi - (nx > 0.0 && fabs(q) < 0.02 ? atan_small(q) : atan2(ny, nx));
     if (php >= TWOPI) php -= TWOPI;
