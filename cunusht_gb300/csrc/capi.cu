@@ -234,6 +234,7 @@ static int build_plan(cunusht_plan_s *P, int lmax, double eps, int precision, in
     P->nph_uniform = (int)P->h_nph[0];
     for (int i = 1; i < nring; ++i)
         if (P->h_nph[i] != P->h_nph[0]) P->nph_uniform = 0;
+    P->ring_shifted = std::any_of(P->h_phi0.begin(), P->h_phi0.end(), [](double p) { return p != 0.0; });
 
     // ring pairs (theta, pi - theta)
     {

@@ -182,6 +182,7 @@ struct cunusht_plan_s {
     int nring = 0;
     long long npix = 0;
     int nph_uniform = 0;  // all rings have this many pixels (0 if not uniform)
+    bool ring_shifted = true;  // a ring starts at phi0 != 0
     std::vector<double> h_theta, h_phi0;
     std::vector<long long> h_nph, h_ofs;
     double *d_ring_theta = nullptr, *d_ring_phi0 = nullptr;

@@ -946,10 +946,12 @@ __device__ __forceinline__ void ring_class(const RingCls &rc, int ring, int &N, 
 // shared memory behind the twiddles (nside 512, lmax 1000, double-float: 1.17
 // -> 0.79 ms; the same sines and cosines), up to 200 KB in all: a table that
 // takes the last of the L1 cache made the 16384-point rings of lmax 4095 8 %
-// slower (4.9 -> 5.3 ms).
-__host__ __device__ inline size_t ring_phase_bytes(int L, size_t sm) {
-    const size_t b = (size_t)(L + 1) * sizeof(double2);
-    return sm + b <= 200 * 1024 ? b : 0;
+// slower (4.9 -> 5.3 ms).  Grids whose rings all start at zero never read it and
+// get none: with it, 512 Gauss-Legendre rings of 1031 pixels (lmax 511) took 0.131
+// ms instead of 0.125, 2048 rings of 4099 pixels 2.17 instead of 2.10.
+static size_t ring_phase_bytes(const cunusht_plan_s *P, size_t sm) {
+    const size_t b = (size_t)(P->lmax + 1) * sizeof(double2);
+    return P->ring_shifted && sm + b <= 200 * 1024 ? b : 0;
 }
 
 template <typename T>
@@ -1474,7 +1476,7 @@ int ring_synth_batch(const cunusht_plan_s *P, int nreq, int spin, const double2 
                      double *out1, long long obs, cudaStream_t st) {
     if (ring_mr_available(P)) return ring_synth_mr_batch(P, nreq, spin, Hgl, hbs, out0, out1, obs, st);
     size_t sm = fft_smem_bytes(ring_buffer_len(P), false);
-    const size_t pb = ring_phase_bytes(P->lmax, sm);
+    const size_t pb = ring_phase_bytes(P, sm);
     const int ptab_len = (int)(pb / sizeof(double2));
     sm += pb;
     dim3 grid(P->nring, nreq);

@@ -192,6 +192,7 @@ extern "C" int cunusht_synthesis_noalloc(int lmax, int spin, int ncomp, const vo
         ++np;
     }
     for (int i = 0; i < nring; ++i) R.phi0[i] = ring_phi0[i];
+    P.ring_shifted = std::any_of(ring_phi0, ring_phi0 + nring, [](double p) { return p != 0.0; });
     P.gl_npairs = np;
     int Mb = 1;
     while (Mb < 2 * nphi - 1) Mb <<= 1;
