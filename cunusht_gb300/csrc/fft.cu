@@ -123,14 +123,19 @@ __device__ __forceinline__ cplx<T> tw_quarter(const cplx<T> *S, int t, int lq) {
     return mk<T>(x, y);
 }
 
-// Product with a twiddle. FP32: fixed fused operations, the ones the compiler
-// makes of cmul in fft_pass_e, so that passes joined in registers round alike.
+// Product with a twiddle in every pass.  FP32 and FP64: fixed fused operations,
+// so that passes joined in registers round as the single passes do, whatever
+// the compiler would contract of cmul in each (a 2048-point FP64 transform
+// differed between the block sizes).
 template <typename C> __device__ __forceinline__ C tw_mul(C a, C b) { return cmul(a, b); }
 __device__ __forceinline__ float2 tw_mul(float2 a, float2 b) {
     return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
+__device__ __forceinline__ double2 tw_mul(double2 a, double2 b) {
+    return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
 
-template <typename T, int R, int NB, bool SMALL = false>
+template <typename T, int R, int NB>
 __device__ __forceinline__ void fft_pass_e(cplx<T> *buf, int N, int Ns, int dir,
                                            const cplx<T> *__restrict__ stw, int M, int nthr) {
     using C = cplx<T>;
@@ -158,7 +163,7 @@ __device__ __forceinline__ void fft_pass_e(cplx<T> *buf, int N, int Ns, int dir,
                 for (int r = 1; r < R; ++r) {
                     C w = tw_quarter<T>(stw, r * k * tstep, lq);
                     if (dir > 0) w.y = -w.y;
-                    v[c][r] = SMALL ? tw_mul(v[c][r], w) : cmul(v[c][r], w);
+                    v[c][r] = tw_mul(v[c][r], w);
                 }
             }
             dftR<T, R>(v[c], dir);
@@ -386,8 +391,8 @@ template <typename T>
 __device__ __forceinline__ void fft_tail2(cplx<T> *buf, int N, int Ns, int dir, const cplx<T> *__restrict__ stw, int M,
                                           int rem) {
     for (; rem > 0; --rem, Ns <<= 1) {
-        if (N > 4 * FFT_SMALL_TPB) fft_pass_e<T, 2, 4, true>(buf, N, Ns, dir, stw, M, N / 8);
-        else fft_pass_e<T, 2, 2, true>(buf, N, Ns, dir, stw, M, N / 4);
+        if (N > 4 * FFT_SMALL_TPB) fft_pass_e<T, 2, 4>(buf, N, Ns, dir, stw, M, N / 8);
+        else fft_pass_e<T, 2, 2>(buf, N, Ns, dir, stw, M, N / 4);
     }
 }
 
@@ -404,8 +409,8 @@ __device__ __forceinline__ void fft_smem_small(cplx<T> *buf, int N, int dir, con
         constexpr int nthr = FFT_SMALL_TPB;
         for (; rem >= 4; rem -= 4, Ns <<= 4) fft_pass16<T>(buf, N, Ns, dir, stw, M, nthr);
         if (rem == 3) fft_pass8<T>(buf, N, Ns, dir, stw, M, nthr);
-        else if (rem == 2) fft_pass_e<T, 4, 4, true>(buf, N, Ns, dir, stw, M, nthr);
-        else if (rem == 1) fft_pass_e<T, 2, 8, true>(buf, N, Ns, dir, stw, M, nthr);
+        else if (rem == 2) fft_pass_e<T, 4, 4>(buf, N, Ns, dir, stw, M, nthr);
+        else if (rem == 1) fft_pass_e<T, 2, 8>(buf, N, Ns, dir, stw, M, nthr);
         return;
     }
     for (; rem >= 3; rem -= 3, Ns <<= 3) fft_pass2s<T, 3>(buf, N, Ns, dir, stw, M);

@@ -790,7 +790,7 @@ int nufft_spread(const cunusht_plan_s *P, int spin, const double *loc, long long
 // difference (equal modulo 2 pi).
 // geo (may be NULL): per ring sin, cos, cot of the colatitude and the pixel spacing, from the plan.
 // FP64 instructions bound it: about 330 per pixel with sincos, three atan2 and the divisions by
-// constants, about 100 with ring tables and series of the increments; 8.4 M pixels 4.46 -> 1.31 ms.
+// constants, about 100 with ring tables and series of the increments; 8.4 M pixels 4.46 -> 1.35 ms.
 __device__ __forceinline__ double asin_small(double x) {  // |x| < 0.02: error below 1e-20
     const double x2 = x * x;
     return x + x * x2 * (1.0 / 6.0 + x2 * (3.0 / 40.0 + x2 * (15.0 / 336.0 + x2 * (105.0 / 3456.0))));
