@@ -638,6 +638,15 @@ int cunusht_plan_set_tensor_cores(cunusht_plan_t *P, int enable) {
     return CUNUSHT_OK;
 }
 
+int cunusht_plan_set_wait_limit(cunusht_plan_t *P, int polls) {
+    clear_error();
+    RC_TRY(check_plan(P));
+    ARG_CHECK(P->prec == CUNUSHT_PREC_FP64, "the wait limit belongs to FP64 plans");
+    ARG_CHECK(polls >= 0 && polls <= 1 << 22, "polls must be in [0, 2^22], got %d", polls);
+    P->wait_limit = polls;
+    return CUNUSHT_OK;
+}
+
 int cunusht_plan_device_status(cunusht_plan_t *P, int *status) {
     clear_error();
     RC_TRY(check_plan(P));

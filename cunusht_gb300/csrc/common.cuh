@@ -220,6 +220,7 @@ struct cunusht_plan_s {
     int *d_tc_woff[3] = {};   // first window of each m (m = 0..lmax+1)
     bool use_tc = true;       // Legendre stages (every spin) on the tensor cores
     int *d_status = nullptr;  // device status word: bit 0 = a bounded wait of a tensor-core kernel ran out
+    int wait_limit = 1 << 22;  // polls of each wait of the FP64 plans' kernels (tests set 0: every wait runs out)
     // tensor-core synthesis: record buffer (alm digit planes and scales per (m, l-window), written per call)
     unsigned char *d_tc_rec = nullptr;
     size_t tc_rec_bytes = 0;

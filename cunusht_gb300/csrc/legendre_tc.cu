@@ -509,6 +509,7 @@ __global__ void __launch_bounds__(TclLayout<NB>::BLOCK, TclLayout<NB>::BPS)
     const int kw0 = work ? cb / CPW : 0, cs0 = cb - kw0 * CPW;
     if (tid == 0 && work) fetch(kw0, 0);
 
+    int issued = 0;  // chunks whose MMAs the MMA warp has issued
     if (warp == T / 32) {
         // ---------------- MMA warp: the whole warp follows the chunk sequence (its
         // outcome kept warp-uniform), lane 0 issues
@@ -541,8 +542,7 @@ __global__ void __launch_bounds__(TclLayout<NB>::BLOCK, TclLayout<NB>::BPS)
                 __syncwarp();
             }
         }
-        if (!ok && gc > 0) mbar_wait(empty0 + 8 * ((gc - 1) & 1), ((gc - 1) >> 1) & 1);
-        __syncwarp();
+        issued = gc;
     } else {
         // ---------------- ring warps
         const int tile = tid >> 7, row = tid & 127;
@@ -687,7 +687,8 @@ __global__ void __launch_bounds__(TclLayout<NB>::BLOCK, TclLayout<NB>::BPS)
             *s_bad = 1;
             if (tid == 0) {
                 if (status) atomicOr(status, 1);
-                // the record copy of the window after the last one entered may still be in flight
+                // the record copies of the last window entered and of the one after it may still be in flight
+                mbar_wait(rbar0 + 8 * (kl & 1), (kl >> 1) & 1);
                 if (l0 + (kw + 1) * TCL_W <= L) mbar_wait(rbar0 + 8 * ((kl + 1) & 1), ((kl + 1) >> 1) & 1);
             }
         } else if (act && S0) {
@@ -726,6 +727,9 @@ __global__ void __launch_bounds__(TclLayout<NB>::BLOCK, TclLayout<NB>::BPS)
     tc_fence_before();
     __syncthreads();
     if (warp == T / 32) {
+        // after a wait that ran out, wherever it did, the MMAs issued may still be in flight
+        if (*s_bad && issued > 0) mbar_wait(empty0 + 8 * ((issued - 1) & 1), ((issued - 1) >> 1) & 1);
+        __syncwarp();
         tc_fence_after();
         tmem_dealloc(tbase, LY::NCOLS);
     }

@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
     k_leg_synth_tc64(int L, int spin, const unsigned char *__restrict__ rec, const int *__restrict__ woff,
                      const double2 *__restrict__ lg0, int npairs, const double *__restrict__ px,
                      const RingLog *__restrict__ lsc, const int *__restrict__ prn, const int *__restrict__ prs, const double2 *__restrict__ stv, const short2 *__restrict__ ste,
-                     int st_ld, const short *__restrict__ es, double2 *__restrict__ H, int ldH, int *status) {
+                     int st_ld, const short *__restrict__ es, double2 *__restrict__ H, int ldH, int wlim, int *status) {
     constexpr int T = T6_T;
     extern __shared__ __align__(1024) unsigned char sm[];
     uint32_t *s_tm = reinterpret_cast<uint32_t *>(sm + T6_OFF_TM);
@@ -381,6 +381,7 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
     const int kw0 = work ? cb / T6_CPW : 0, cs0 = cb - kw0 * T6_CPW;
     if (tid == 0 && work) bulk_g2s(sbase + T6_OFF_R, recm + (size_t)kw0 * T6_RSZ, T6_RSZ, rbar0);
 
+    int issued = 0;  // chunks whose MMAs the MMA warp has issued
     if (warp == T / 32) {
         // ---------------- MMA warp: follows the chunk sequence (outcome warp-uniform), lane 0 issues
         constexpr uint32_t IDESC = idesc_f16_f32(128, T6_NN);
@@ -392,7 +393,7 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
             const int cs = kw == kw0 ? cs0 : 0;
             for (int c = cs; c < nch; ++c, ++gc) {
                 const int buf = gc & 1;
-                const bool got = !*s_bad && mbar_wait(full0 + 8 * buf, (gc >> 1) & 1);
+                const bool got = !*s_bad && mbar_wait(full0 + 8 * buf, (gc >> 1) & 1, wlim);
                 if (!__all_sync(0xffffffffu, got)) {
                     *s_bad = 1;
                     ok = false;
@@ -412,8 +413,7 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
                 __syncwarp();
             }
         }
-        if (!ok && gc > 0) mbar_wait(empty0 + 8 * ((gc - 1) & 1), ((gc - 1) >> 1) & 1);
-        __syncwarp();
+        issued = gc;
     } else {
         // ---------------- ring warps
         const int tile = tid >> 7, row = tid & 127;
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
                 bulk_g2s(sbase + T6_OFF_R + ((kl + 1) & 1) * T6_RSZ, recm + (size_t)(kw + 1) * T6_RSZ, T6_RSZ,
                          rbar0 + 8 * ((kl + 1) & 1));
             }
-            bad |= !mbar_wait(rbar0 + 8 * (kl & 1), (kl >> 1) & 1);
+            bad |= !mbar_wait(rbar0 + 8 * (kl & 1), (kl >> 1) & 1, wlim);
             const unsigned char *Rw = sm + T6_OFF_R + (kl & 1) * T6_RSZ;
             const unsigned short *s_tp = reinterpret_cast<const unsigned short *>(Rw);
             const double *s_sc = reinterpret_cast<const double *>(Rw + T6_RSC);
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
             for (int c = kw == kw0 ? cs0 : 0; c < nch; ++c, ++gc) {
                 const int buf = gc & 1;
                 const bool live = kw * T6_CPW + c >= 2 * c_me;
-                if (gc >= 2) bad |= !mbar_wait(empty0 + 8 * buf, ((gc - 2) >> 1) & 1);
+                if (gc >= 2) bad |= !mbar_wait(empty0 + 8 * buf, ((gc - 2) >> 1) & 1, wlim);
                 unsigned char *sA = sm + buf * T6_ABUF;
                 unsigned char *sB = sm + T6_OFF_B + buf * T6_BBUF;
                 if (b_dst >= 0)
@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
                 if (lane == 0) mbar_arrive(full0 + 8 * buf);
             }
             // window epilogue: column n = g NO + o holds the exact sum of weight 2^-8g, |sum| < 2^24
-            bad |= !mbar_wait(empty0 + 8 * ((gc - 1) & 1), ((gc - 1) >> 1) & 1);
+            bad |= !mbar_wait(empty0 + 8 * ((gc - 1) & 1), ((gc - 1) >> 1) & 1, wlim);
             bad = __any_sync(0xffffffffu, bad);
             tc_fence_after();
             if (!bad) {
@@ -573,7 +573,8 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
             *s_bad = 1;
             if (tid == 0) {
                 if (status) atomicOr(status, 1);
-                // the record copy of the window after the last one entered may still be in flight
+                // the record copies of the last window entered and of the one after it may still be in flight
+                mbar_wait(rbar0 + 8 * (kl & 1), (kl >> 1) & 1);
                 if (l0 + (kw + 1) * T6_W <= L) mbar_wait(rbar0 + 8 * ((kl + 1) & 1), ((kl + 1) >> 1) & 1);
             }
         } else if (act) {
@@ -597,6 +598,9 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
     tc_fence_before();
     __syncthreads();
     if (warp == T / 32) {
+        // after a wait that ran out, wherever it did, the MMAs issued may still be in flight
+        if (*s_bad && issued > 0) mbar_wait(empty0 + 8 * ((issued - 1) & 1), ((issued - 1) >> 1) & 1);
+        __syncwarp();
         tc_fence_after();
         tmem_dealloc(tbase, T6_NT * T6_NN);
     }
@@ -734,7 +738,7 @@ int leg_synth_tc64(const cunusht_plan_s *P, int npairs, const double *x, const d
         CU_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T6_BYTES));
         kern<<<dim3((ntc + per - 1) / per, P->mmax + 1), T6_BLOCK, T6_BYTES, st>>>(
             L, spin, P->d_t6_rec, P->d_t6_woff[spin], P->d_t6_lg0[spin], ntc, x, lsc, rn, rs, stv, ste, st_ld,
-            P->d_t6_es[spin], H, ld, P->d_status);
+            P->d_t6_es[spin], H, ld, P->wait_limit, P->d_status);
         CU_LAUNCH_CHECK();
         return CUNUSHT_OK;
     };

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
                    const int *__restrict__ woff, const double2 *__restrict__ lg0, int npairs,
                    const double *__restrict__ px, const RingLog *__restrict__ lsc, const int *__restrict__ prn,
                    const int *__restrict__ prs, const double2 *__restrict__ stv, const short2 *__restrict__ ste,
-                   int st_ld, double *__restrict__ Gout, double *__restrict__ Cout, int *status) {
+                   int st_ld, double *__restrict__ Gout, double *__restrict__ Cout, int wlim, int *status) {
     extern __shared__ __align__(1024) unsigned char sm[];
     uint32_t *s_tm = reinterpret_cast<uint32_t *>(sm + A6_OFF_MISC);
     volatile int *s_bad = reinterpret_cast<volatile int *>(sm + A6_OFF_MISC + 4);
@@ -179,17 +179,16 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
     const int lstart = cb < nchk ? l0 + A6_KC * cb : L + 1;
     const short *ebm = eb + 8 * (long long)woff[m];  // El per chunk
 
+    int issued = 0;  // chunks whose MMAs the MMA warp has issued
     if (warp == A6_MMA) {
         constexpr uint32_t IDESC = idesc_f16_f32(128, A6_NN) | (1u << 15) | (1u << 16);  // A, B MN-major
         int gc = 0;
-        bool ok = true;
         for (int lb = lstart; lb <= L; lb += A6_KC, ++gc) {
             const int buf = gc & 1, tb = gc % A6_NTB;
-            bool got = !*s_bad && mbar_wait(bfull0 + 8 * buf, (gc >> 1) & 1);
-            if (got && gc >= A6_NTB) got = mbar_wait(tempty0 + 8 * tb, ((gc / A6_NTB) - 1) & 1);
+            bool got = !*s_bad && mbar_wait(bfull0 + 8 * buf, (gc >> 1) & 1, wlim);
+            if (got && gc >= A6_NTB) got = mbar_wait(tempty0 + 8 * tb, ((gc / A6_NTB) - 1) & 1, wlim);
             if (!__all_sync(0xffffffffu, got)) {
                 *s_bad = 1;
-                ok = false;
                 break;
             }
             if (lane == 0) {
@@ -204,8 +203,7 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
             }
             __syncwarp();
         }
-        if (!ok && gc > 0) mbar_wait(bempty0 + 8 * ((gc - 1) & 1), ((gc - 1) >> 1) & 1);
-        __syncwarp();
+        issued = gc;
     } else if (epi) {
         // lane = row (digit j = lane / 4, column lane % 4); rows 28 .. 31 are zero
         const int eh = warp >> 2, j = lane >> 2, col = lane & 3;
@@ -214,7 +212,7 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
         int gc = 0;
         for (int lb = lstart; lb <= L; lb += A6_KC, ++gc) {
             const int tb = gc % A6_NTB;
-            const bool got = !*s_bad && mbar_wait(tfull0 + 8 * tb, (gc / A6_NTB) & 1);
+            const bool got = !*s_bad && mbar_wait(tfull0 + 8 * tb, (gc / A6_NTB) & 1, wlim);
             if (!__all_sync(0xffffffffu, got)) {
                 *s_bad = 1;
                 break;
@@ -292,7 +290,7 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
         int gc = 0, bad = 0;
         for (int lb = lstart; lb <= L; lb += A6_KC, ++gc) {
             const int buf = gc & 1, ck = (lb - l0) / A6_KC;
-            if (gc >= 2) bad |= !mbar_wait(bempty0 + 8 * buf, ((gc - 2) >> 1) & 1);
+            if (gc >= 2) bad |= !mbar_wait(bempty0 + 8 * buf, ((gc - 2) >> 1) & 1, wlim);
             bad = __any_sync(0xffffffffu, bad | *s_bad);
             if (bad) break;
             unsigned char *sB = sm + A6_OFF_B + buf * A6_BBUF + boff;
@@ -385,6 +383,9 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
     __syncthreads();
     if (tid == 0 && *s_bad && status) atomicOr(status, 1);
     if (warp == A6_MMA) {
+        // after a wait that ran out, wherever it did, the MMAs issued may still be in flight
+        if (*s_bad && issued > 0) mbar_wait(bempty0 + 8 * ((issued - 1) & 1), ((issued - 1) >> 1) & 1);
+        __syncwarp();
         tc_fence_after();
         tmem_dealloc(tbase, 512);
     }
@@ -412,7 +413,7 @@ int leg_adjoint_tc64(const cunusht_plan_s *P, int npairs, const double *x, const
         CU_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, A6_BYTES));
         kern<<<dim3((ntc + per - 1) / per, P->mmax + 1), A6_THREADS, A6_BYTES, st>>>(
             L, spin, ncomp, H, ld, lf, P->d_t6_ag[spin], P->d_t6_fx[spin], P->d_t6_cl[spin], P->d_t6_eb[spin],
-            P->d_t6_es[spin], P->d_t6_woff[spin], P->d_t6_lg0[spin], ntc, x, lsc, rn, rs, stv, ste, st_ld, (double *)G, (double *)C, P->d_status);
+            P->d_t6_es[spin], P->d_t6_woff[spin], P->d_t6_lg0[spin], ntc, x, lsc, rn, rs, stv, ste, st_ld, (double *)G, (double *)C, P->wait_limit, P->d_status);
         CU_LAUNCH_CHECK();
         return CUNUSHT_OK;
     };

@@ -270,18 +270,17 @@ __global__ void __launch_bounds__(TCA_THREADS, 1)
     const int cb = *s_c0;
     const int lstart = cb < nchk ? l0 + TCA_KC * cb : L + 1;
 
+    int issued = 0;  // chunks whose MMAs the MMA warp has issued
     if (warp == TCA_MMA) {
         // ---------------- MMA warp
         constexpr uint32_t IDESC = idesc_bf16_f32(128, 4 * TCA_KC) | (1u << 15) | (1u << 16);  // A, B MN-major
         int gc = 0;
-        bool ok = true;
         for (int lb = lstart; lb <= L; lb += TCA_KC, ++gc) {
             const int buf = gc & 1, tb = gc % TCA_NTB;
             bool got = !*s_bad && mbar_wait(bfull0 + 8 * buf, (gc >> 1) & 1);
             if (got && gc >= TCA_NTB) got = mbar_wait(tempty0 + 8 * tb, ((gc / TCA_NTB) - 1) & 1);
             if (!__all_sync(0xffffffffu, got)) {
                 *s_bad = 1;
-                ok = false;
                 break;
             }
             if (lane == 0) {
@@ -296,8 +295,7 @@ __global__ void __launch_bounds__(TCA_THREADS, 1)
             }
             __syncwarp();
         }
-        if (!ok && gc > 0) mbar_wait(bempty0 + 8 * ((gc - 1) & 1), ((gc - 1) >> 1) & 1);
-        __syncwarp();
+        issued = gc;
     } else if (warp >= TCA_EPI0) {
         // ---------------- epilogue warps: TMEM lane quarter q = warp % 4, row 32 q + lane
         const int q = warp & 3, row = 32 * q + lane, eid = tid - TCA_EPI0 * 32;
@@ -414,6 +412,9 @@ __global__ void __launch_bounds__(TCA_THREADS, 1)
     __syncthreads();
     if (tid == 0 && *s_bad && status) atomicOr(status, 1);
     if (warp == TCA_MMA) {
+        // after a wait that ran out, wherever it did, the MMAs issued may still be in flight
+        if (*s_bad && issued > 0) mbar_wait(bempty0 + 8 * ((issued - 1) & 1), ((issued - 1) >> 1) & 1);
+        __syncwarp();
         tc_fence_after();
         tmem_dealloc(tbase, TCA_TCOLS);
     }

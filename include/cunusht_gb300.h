@@ -178,6 +178,14 @@ int cunusht_plan_set_spreading(cunusht_plan_t *plan, int method, int determinist
 int cunusht_plan_device_status(cunusht_plan_t *plan, int *status);
 
 /*
+ * Polls after which a bounded wait of an FP64 plan's tensor-core kernels runs
+ * out (2^22 by default).  0: every wait runs out at once, as if nothing ever
+ * arrived -- for tests of what a call then does; the context stays usable.  No
+ * reference counterpart.
+ */
+int cunusht_plan_set_wait_limit(cunusht_plan_t *plan, int polls);
+
+/*
  * Tensor-core self test: a 128 x n x 32 product of integer matrices
  * (n = 16, 32 or 64, entries |.| <= 128) accumulated reps times (1..16, sums
  * below 2^24) through the descriptors, tensor-memory accumulation and
