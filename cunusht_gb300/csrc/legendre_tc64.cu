@@ -38,8 +38,8 @@
 // full (one arrival per ring warp) and empty (commit) mbarriers; the window
 // records (k_tc64_records) arrive by bulk copy, the next one prefetched.
 // Every wait is bounded; a block whose wait runs out sets bit 0 of the plan's
-// status word, waits once more for its own copies and MMAs, frees its tensor
-// memory and returns.
+// status word, writes NaN to its rings (no caller polls that word), waits once
+// more for its own copies and MMAs, frees its tensor memory and returns.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "rec64.cuh"
@@ -577,7 +577,11 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
                 mbar_wait(rbar0 + 8 * (kl & 1), (kl >> 1) & 1);
                 if (l0 + (kw + 1) * T6_W <= L) mbar_wait(rbar0 + 8 * ((kl + 1) & 1), ((kl + 1) >> 1) & 1);
             }
-        } else if (act) {
+            // H holds an earlier call's columns: nothing may pass for this one's
+#pragma unroll
+            for (int o = 0; o < T6_NO; ++o) acc[o] = nan("");
+        }
+        if (act) {
             const int n = prn[p], s = prs[p];
             if (S0) {
                 H[(long long)m * ldH + n] = make_double2(acc[0] + acc[2], acc[1] + acc[3]);

@@ -24,7 +24,8 @@
 // the tensor-memory lanes 32 (warp mod 4) .. + 31, and the used rows are lanes
 // 0 .. 27).  Two B buffers and four tensor-memory buffers with full / empty
 // mbarriers.  Every wait is bounded; on a timeout the block sets bit 0 of the
-// plan's status word and returns.
+// plan's status word, makes the order's alm NaN (no caller polls that word) and
+// returns.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "rec64.cuh"
@@ -54,6 +55,14 @@ static_assert(A6_BYTES <= 227 * 1024, "dynamic shared memory of one block");
 static_assert(A6_BBUF % 1024 == 0 && A6_OFF_BAR % 8 == 0, "layout alignment");
 
 __device__ __forceinline__ long long shfl_xor_ll(long long v, int mask) { return __shfl_xor_sync(0xffffffffu, v, mask); }
+
+// n alm from entry i0 on become NaN, whatever other blocks add
+__device__ __noinline__ void add_nan(double *G, double *C, long long i0, int n, int t, int nt) {
+    for (int i = t; i < 2 * n; i += nt) {
+        atomicAdd(G + 2 * i0 + i, nan(""));
+        if (C) atomicAdd(C + 2 * i0 + i, nan(""));
+    }
+}
 
 template <bool S0>
 __global__ void __launch_bounds__(A6_THREADS, 1)
@@ -381,7 +390,10 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
     }
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && *s_bad && status) atomicOr(status, 1);
+    if (*s_bad) {  // the block's part of the sums is missing
+        if (tid == 0 && status) atomicOr(status, 1);
+        add_nan(Gout, !S0 && ncomp > 1 ? Cout : nullptr, b + l0, L + 1 - l0, tid, A6_THREADS);
+    }
     if (warp == A6_MMA) {
         // after a wait that ran out, wherever it did, the MMAs issued may still be in flight
         if (*s_bad && issued > 0) mbar_wait(bempty0 + 8 * ((issued - 1) & 1), ((issued - 1) >> 1) & 1);

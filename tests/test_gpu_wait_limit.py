@@ -58,3 +58,21 @@ def test_block_that_gives_up_waits_for_its_own_copies(built_lib, lmax, spin):
             x = call()
             assert float((x - ref).norm() / ref.norm()) < 2.0 ** -50, name
         assert _status(t) == 0
+
+
+# ring counts without a short tail, whose rings go to the CUDA cores
+@pytest.mark.parametrize("lmax", [100, 400, 600])
+@pytest.mark.parametrize("spin", [0, 2])
+def test_results_of_a_block_that_gives_up_are_not_numbers(built_lib, lmax, spin):
+    """Every pixel and every alm (l >= spin) is NaN, also after a call that left
+    its numbers in the plan's buffers, and none in the call after it."""
+    t = _plan(lmax)
+    valid = torch.cat([torch.arange(m, lmax + 1) for m in range(lmax + 1)]).cuda() >= spin
+    for name, call in _calls(t, lmax, spin):
+        call()
+        _limit(t, 0)
+        x = call()
+        assert _status(t) == 1
+        assert bool(torch.isnan(x[..., valid] if x.is_complex() else x).all()), name
+        _limit(t, 1 << 22)
+        assert bool(torch.isfinite(call()).all()), name
