@@ -427,6 +427,13 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
         const long long rnd = idle ? 0 : FIX_ROUND;
         bool fixed = false;
         const bool may_fix = __any_sync(0xffffffffu, !idle);
+        // windows before the block's first: no digits, but a value in them that is not finite (scale NaN) counts
+        bool nonfin = false;
+        for (int k = lane; k < (work ? kw0 : woff[m + 1] - woff[m]); k += 32) {
+            const double *sc = reinterpret_cast<const double *>(recm + (size_t)k * T6_RSZ + T6_RSC);
+            nonfin |= isnan(sc[0] + sc[1] + sc[2] + sc[3]);
+        }
+        nonfin = __any_sync(0xffffffffu, nonfin);
         const uint32_t t_lane = tbase + ((uint32_t)((warp & 3) * 32) << 16) + tile * T6_NN;
         const uint32_t a_row = (uint32_t)tile * T6_TILE + (row >> 3) * T6_SBO + (row & 7) * 16;
         // this thread's B' copy: row n = g NO + o, K-core di = t_{g-di} of output o (28 pairs x 4 outputs)
@@ -577,7 +584,8 @@ __global__ void __launch_bounds__(T6_BLOCK, 2)
                 mbar_wait(rbar0 + 8 * (kl & 1), (kl >> 1) & 1);
                 if (l0 + (kw + 1) * T6_W <= L) mbar_wait(rbar0 + 8 * ((kl + 1) & 1), ((kl + 1) >> 1) & 1);
             }
-            // H holds an earlier call's columns: nothing may pass for this one's
+        }
+        if (bad || nonfin) {  // H holds an earlier call's columns: after a wait that ran out nothing may pass for this one's
 #pragma unroll
             for (int o = 0; o < T6_NO; ++o) acc[o] = nan("");
         }

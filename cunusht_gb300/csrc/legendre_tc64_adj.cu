@@ -186,6 +186,9 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
     const int nchk = l0 <= L ? (L - l0 + A6_KC) / A6_KC : 0;
     const int cb = *s_c0;
     const int lstart = cb < nchk ? l0 + A6_KC * cb : L + 1;
+    // the l before it get no digit products, but a column that is not finite makes them NaN as well
+    if (lstart > l0 && max(max(s_ea[0], s_ea[1]), max(s_ea[2], s_ea[3])) == 1025)
+        add_nan(Gout, !S0 && ncomp > 1 ? Cout : nullptr, b + l0, lstart - l0, tid, A6_THREADS);
     const short *ebm = eb + 8 * (long long)woff[m];  // El per chunk
 
     int issued = 0;  // chunks whose MMAs the MMA warp has issued
