@@ -91,13 +91,13 @@ int leg_synth_pole_pair(const cunusht_plan_s *P, int nreq, int spin, const doubl
                         cudaStream_t st);
 // legendre_tc64.cu: tensor-core synthesis of the FP64 plans (one request)
 int tc64_plan_init(cunusht_plan_s *P);
-int leg_synth_tc64(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
-                   const int *rn, const int *rs, int ld, int pole, int pole_rn, int pole_rs, bool cc, int spin,
-                   const double2 *G, const double2 *C, const double *lf, double2 *H, cudaStream_t st);
+int leg_synth_tc64(const cunusht_plan_s *P, int npairs, const double *x, const int *rn, const int *rs, int ld,
+                   int pole, int pole_rn, int pole_rs, bool cc, int spin, const double2 *G, const double2 *C,
+                   const double *lf, double2 *H, cudaStream_t st);
 // legendre_tc64_adj.cu: tensor-core adjoint of the FP64 plans (one request, alm zeroed by the caller)
-int leg_adjoint_tc64(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
-                     const int *rn, const int *rs, int ld, int pole, int pole_rn, int pole_rs, bool cc, int spin,
-                     int ncomp, const double2 *H, const double *lf, double2 *G, double2 *C, cudaStream_t st);
+int leg_adjoint_tc64(const cunusht_plan_s *P, int npairs, const double *x, const int *rn, const int *rs, int ld,
+                     int pole, int pole_rn, int pole_rs, bool cc, int spin, int ncomp, const double2 *H,
+                     const double *lf, double2 *G, double2 *C, cudaStream_t st);
 int leg_adj_f64_pairs(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
                       const int *rn, const int *rs, int ld, int spin, int ncomp, const double2 *H, const double *lf,
                       double2 *G, double2 *C, cudaStream_t st);

@@ -1161,8 +1161,8 @@ int leg_synth_batch_fl(const cunusht_plan_s *P, int nreq, int spin, const double
         const double2 *Gr = G + r * astride, *Cr = C ? C + r * astride : nullptr;
         double2 *Hr = H + r * hstride;
         if (f64_tensor_cores(P, spin))
-            RC_TRY(leg_synth_tc64(P, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.ld, R.pole, R.pole_rn, R.pole_rs, cc,
-                                  spin, Gr, Cr, lf, Hr, st));
+            RC_TRY(leg_synth_tc64(P, R.npairs, R.x, R.rn, R.rs, R.ld, R.pole, R.pole_rn, R.pole_rs, cc, spin, Gr, Cr,
+                                  lf, Hr, st));
         else
             RC_TRY(leg_synth_f64_pairs(P, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.ld, spin, Gr, Cr, lf, Hr, st));
     }
@@ -1323,8 +1323,8 @@ int leg_adjoint_batch(const cunusht_plan_s *P, int nreq, int spin, int ncomp, co
         const double2 *Hr = H + r * hstride;
         double2 *Gr = G + r * astride, *Cr = (spin > 0 && ncomp > 1) ? C + r * astride : nullptr;
         if (f64_tensor_cores(P, spin))
-            RC_TRY(leg_adjoint_tc64(P, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.ld, R.pole, R.pole_rn, R.pole_rs, cc,
-                                    spin, ncomp, Hr, lf, Gr, Cr, st));
+            RC_TRY(leg_adjoint_tc64(P, R.npairs, R.x, R.rn, R.rs, R.ld, R.pole, R.pole_rn, R.pole_rs, cc, spin, ncomp,
+                                    Hr, lf, Gr, Cr, st));
         else
             RC_TRY(leg_adj_f64_pairs(P, R.npairs, R.x, R.sh, R.ch, R.rn, R.rs, R.ld, spin, ncomp, Hr, lf, Gr, Cr,
                                      st));

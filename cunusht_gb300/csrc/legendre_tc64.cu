@@ -78,7 +78,6 @@ constexpr int T6_OFF_R = T6_OFF_B + 2 * T6_BBUF;
 constexpr int T6_OFF_BAR = T6_OFF_R + 2 * T6_RSZ;   // full[2], empty[2], record[2]
 constexpr int T6_OFF_TM = T6_OFF_BAR + 48;          // tensor-memory base, give-up flag, first chunk
 constexpr int T6_BYTES = T6_OFF_TM + 16;
-constexpr int T6_MIN_TAIL = 32;           // fewer leftover ring pairs go to the CUDA-core kernel
 static_assert(T6_BYTES <= 227 * 1024, "dynamic shared memory of one block");
 static_assert(T6_RCO % 16 == 0 && T6_RSZ % 16 == 0 && T6_OFF_R % 16 == 0, "bulk copies on 16 bytes");
 static_assert(T6_OFF_BAR % 8 == 0, "mbarriers are 8-byte words");
@@ -725,40 +724,38 @@ int tc64_plan_init(cunusht_plan_s *P) {
     return CUNUSHT_OK;
 }
 
-// Ring pairs [0, return value) of a grid done on the tensor cores (after the
-// pole pair, in closed form): all of them, or whole blocks when fewer than
-// T6_MIN_TAIL would be left over.
-int leg_synth_tc64(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
-                   const int *rn, const int *rs, int ld, int pole, int pole_rn, int pole_rs, bool cc, int spin,
-                   const double2 *G, const double2 *C, const double *lf, double2 *H, cudaStream_t st) {
+// One request's synthesis: the pole pair in closed form, every other pair on the
+// tensor cores.  A last block with few rings costs less than the same rings on
+// the CUDA cores, where one warp per order waits on the FP64 pipe for every l
+// (fewer than 32 pairs there: spin 0, 514 pairs, lmax 1026 2.34 ms instead of 1.27,
+// 1540 pairs 27.8 instead of 20.5; spin 2, 258 pairs 1.26 instead of 0.41, 1026
+// pairs 21.0 instead of 12.1).
+int leg_synth_tc64(const cunusht_plan_s *P, int npairs, const double *x, const int *rn, const int *rs, int ld,
+                   int pole, int pole_rn, int pole_rs, bool cc, int spin, const double2 *G, const double2 *C,
+                   const double *lf, double2 *H, cudaStream_t st) {
     const double2 *stv = P->d_t6_stv[cc ? 1 : 0][spin];
     const short2 *ste = P->d_t6_ste[cc ? 1 : 0][spin];
     const RingLog *lsc = P->d_t6_lsc[cc ? 1 : 0];
     const int st_ld = npairs, L = P->lmax;
     if (pole == 0 && npairs > 1) {
         RC_TRY(leg_synth_pole_pair(P, 1, spin, G, C, 0, lf, pole_rn, pole_rs, H, 0, ld, st));
-        ++x, ++sh, ++ch, ++rn, ++rs, ++lsc;
+        ++x, ++rn, ++rs, ++lsc;
         if (stv) ++stv, ++ste;
         --npairs;
     }
-    const int per = spin == 0 ? T6_T : T6_T / 2, tail = npairs % (spin == 0 ? 512 : 256);
-    const int ntc = (npairs > per && tail < T6_MIN_TAIL) ? npairs - tail : npairs;
+    const int per = spin == 0 ? T6_T : T6_T / 2;
     k_tc64_records<<<dim3((L - spin + T6_W) / T6_W, P->mmax + 1), T6_W, 0, st>>>(
         L, spin, G, C, lf, P->d_t6_ag[spin], P->d_t6_cl[spin], P->d_t6_woff[spin], P->d_t6_rec);
     CU_LAUNCH_CHECK();
     auto launch = [&](auto kern) {
         CU_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T6_BYTES));
-        kern<<<dim3((ntc + per - 1) / per, P->mmax + 1), T6_BLOCK, T6_BYTES, st>>>(
-            L, spin, P->d_t6_rec, P->d_t6_woff[spin], P->d_t6_lg0[spin], ntc, x, lsc, rn, rs, stv, ste, st_ld,
+        kern<<<dim3((npairs + per - 1) / per, P->mmax + 1), T6_BLOCK, T6_BYTES, st>>>(
+            L, spin, P->d_t6_rec, P->d_t6_woff[spin], P->d_t6_lg0[spin], npairs, x, lsc, rn, rs, stv, ste, st_ld,
             P->d_t6_es[spin], H, ld, P->wait_limit, P->d_status);
         CU_LAUNCH_CHECK();
         return CUNUSHT_OK;
     };
-    RC_TRY(spin == 0 ? launch(k_leg_synth_tc64<true>) : launch(k_leg_synth_tc64<false>));
-    if (ntc < npairs)
-        RC_TRY(leg_synth_f64_pairs(P, npairs - ntc, x + ntc, sh + ntc, ch + ntc, rn + ntc, rs + ntc, ld, spin, G, C,
-                                   lf, H, st));
-    return CUNUSHT_OK;
+    return spin == 0 ? launch(k_leg_synth_tc64<true>) : launch(k_leg_synth_tc64<false>);
 }
 
 }  // namespace cunusht

@@ -50,7 +50,6 @@ constexpr int A6_OFF_B = A6_ABYTES;
 constexpr int A6_OFF_BAR = A6_OFF_B + 2 * A6_BBUF;   // bfull[2] bempty[2] tfull[4] tempty[4]
 constexpr int A6_OFF_MISC = A6_OFF_BAR + 12 * 8;     // tmem base, bad flag, first chunk, pad, Ea[4], maxima[8][4]
 constexpr int A6_BYTES = A6_OFF_MISC + 16 + 16 + 8 * 16;
-constexpr int A6_MIN_TAIL = 32;
 static_assert(A6_BYTES <= 227 * 1024, "dynamic shared memory of one block");
 static_assert(A6_BBUF % 1024 == 0 && A6_OFF_BAR % 8 == 0, "layout alignment");
 
@@ -407,36 +406,34 @@ __global__ void __launch_bounds__(A6_THREADS, 1)
 }
 
 // One request's adjoint into G (and C), zeroed by the caller: the pole pair in
-// closed form, the other pairs on the tensor cores, fewer than A6_MIN_TAIL
-// left over after whole blocks on the CUDA cores.
-int leg_adjoint_tc64(const cunusht_plan_s *P, int npairs, const double *x, const double *sh, const double *ch,
-                     const int *rn, const int *rs, int ld, int pole, int pole_rn, int pole_rs, bool cc, int spin,
-                     int ncomp, const double2 *H, const double *lf, double2 *G, double2 *C, cudaStream_t st) {
+// closed form, every other pair on the tensor cores (a last block with few rings
+// costs less than these on the CUDA cores: spin 0, 257 pairs, lmax 512 0.78 ms with
+// them there, 0.42 without, 1300 pairs 24.8 and 19.1; spin 2, 129 pairs 0.52 and
+// 0.15, 898 pairs 21.6 and 12.4).
+int leg_adjoint_tc64(const cunusht_plan_s *P, int npairs, const double *x, const int *rn, const int *rs, int ld,
+                     int pole, int pole_rn, int pole_rs, bool cc, int spin, int ncomp, const double2 *H,
+                     const double *lf, double2 *G, double2 *C, cudaStream_t st) {
     const double2 *stv = P->d_t6_stv[cc ? 1 : 0][spin];
     const short2 *ste = P->d_t6_ste[cc ? 1 : 0][spin];
     const RingLog *lsc = P->d_t6_lsc[cc ? 1 : 0];
     const int st_ld = npairs, L = P->lmax;
     const bool has_pole = pole == 0 && npairs > 1;
     if (has_pole) {
-        ++x, ++sh, ++ch, ++rn, ++rs, ++lsc;
+        ++x, ++rn, ++rs, ++lsc;
         if (stv) ++stv, ++ste;
         --npairs;
     }
-    const int per = spin == 0 ? A6_R : A6_R / 2, tail = npairs % per;
-    const int ntc = (npairs > per && tail < A6_MIN_TAIL) ? npairs - tail : npairs;
+    const int per = spin == 0 ? A6_R : A6_R / 2;
     auto launch = [&](auto kern) {
         CU_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, A6_BYTES));
-        kern<<<dim3((ntc + per - 1) / per, P->mmax + 1), A6_THREADS, A6_BYTES, st>>>(
+        kern<<<dim3((npairs + per - 1) / per, P->mmax + 1), A6_THREADS, A6_BYTES, st>>>(
             L, spin, ncomp, H, ld, lf, P->d_t6_ag[spin], P->d_t6_fx[spin], P->d_t6_cl[spin], P->d_t6_eb[spin],
-            P->d_t6_es[spin], P->d_t6_woff[spin], P->d_t6_lg0[spin], ntc, x, lsc, rn, rs, stv, ste, st_ld, (double *)G, (double *)C, P->wait_limit, P->d_status);
+            P->d_t6_es[spin], P->d_t6_woff[spin], P->d_t6_lg0[spin], npairs, x, lsc, rn, rs, stv, ste, st_ld, (double *)G, (double *)C, P->wait_limit, P->d_status);
         CU_LAUNCH_CHECK();
         return CUNUSHT_OK;
     };
     RC_TRY(spin == 0 ? launch(k_leg_adj_tc64<true>) : launch(k_leg_adj_tc64<false>));
     if (has_pole) RC_TRY(leg_adj_pole_pair(P, 1, spin, ncomp, H, 0, ld, lf, pole_rn, pole_rs, G, C, 0, st));
-    if (ntc < npairs)
-        RC_TRY(leg_adj_f64_pairs(P, npairs - ntc, x + ntc, sh + ntc, ch + ntc, rn + ntc, rs + ntc, ld, spin, ncomp, H,
-                                 lf, G, C, st));
     return CUNUSHT_OK;
 }
 
