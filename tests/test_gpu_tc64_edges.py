@@ -64,3 +64,15 @@ def test_short_last_block(built_lib, spin, lmax):
     assert _rel(x, y) < _tol(lmax)
     x, y = _both(t, lambda: t.adjoint_synthesis(v, spin=spin))
     assert _rel(x, y) < _tol(lmax)
+
+
+@pytest.mark.parametrize("spin", [0, 2])
+def test_lmax_4095(built_lib, spin):
+    """The largest size of the configurations: 32 windows of 128 l, 8 or 16 blocks of rings."""
+    lmax = 4095
+    t = _plan(lmax)
+    a, v = _inputs(t, lmax, spin)
+    x, y = _both(t, lambda: t.synthesis(a, spin=spin))
+    assert _rel(x, y) < _tol(lmax)
+    x, y = _both(t, lambda: t.adjoint_synthesis(v, spin=spin))
+    assert _rel(x, y) < _tol(lmax)
