@@ -28,9 +28,11 @@
 // the products are more accurate than the double-float CUDA-core kernels,
 // which round every product to FP32.
 //
-// The FMA pipe bounds it (about 70 % busy): the recursion and the digit split
-// run in packed FP32 for two l, which halves their issue slots, and with up to
-// 2 requests two blocks of two 128-row MMA tiles share an SM.  One request,
+// FP32 issue bounds it (one request, lmax 1023 spin 2: issue slots 61 %, FMA
+// instructions 46 % of the pipe's rate, a packed one holding it twice as long;
+// first stalls long scoreboard and math pipe throttle): the recursion and the
+// digit split run in packed FP32 for two l, which halves their issue slots, and
+// with up to 2 requests two blocks of two 128-row MMA tiles share an SM.  One request,
 // spin 2, lmax 4095: 50.8 -> 41.2 ms; spin 0, lmax 3087: 15.0 -> 10.5 ms;
 // eight requests at lmax 2047: 9.05 -> 8.26 ms.
 //
@@ -1039,9 +1041,9 @@ int leg_synth_pole_pair(const cunusht_plan_s *P, int nreq, int spin, const doubl
     return CUNUSHT_OK;
 }
 
-// Ring pairs in full blocks (256 pairs, 128 for NB = 8; spin 0: 512 and 256) on the tensor cores; a
-// tail of fewer than TCL_MIN_TAIL pairs after at least one full block goes to
-// the double-float CUDA-core kernel instead of a nearly empty block per order m.
+// Ring pairs in blocks of 128 (spin 0: 256) for NB <= 2, 256 (512) for NB = 4 and 192 (384) for
+// NB = 8 on the tensor cores; a tail of fewer than TCL_MIN_TAIL pairs after a multiple of 256 (512)
+// pairs, of 192 (384) for NB = 8, goes to the double-float CUDA-core kernel.
 int leg_synth_spin_tc(const cunusht_plan_s *P, int nb, int npairs, const double *x, const double *sh,
                       const double *ch, const int *rn, const int *rs, int ld, int pole, int pole_rn, int pole_rs,
                       const float4 *stv, const short2 *ste, int spin, const double2 *G, const double2 *C,

@@ -11,8 +11,7 @@
 //     c_{l-1}, to mu_{l+1} = (a_l x + g_l) mu_l - mu_{l-1}: 2 FP64
 //     instructions per step and ring instead of 3 (c_l goes into the alm), and
 //     past the turning point it runs in 64-bit fixed point without any
-//     (rec64.cuh: 22.8 against 37.1 clocks per step of a warp and SM, digits
-//     included); a warp goes over when all its rings have;
+//     (rec64.cuh); a warp goes over when all its rings have;
 //   * mu and the alm are split into seven 8-bit digits on the integer pipe
 //     (rec64.cuh) and multiplied on the tensor cores,
 //         mu = 2^El 2^-7 sum_i d_i 2^-8i,   c a = 2^Ea 2^-7 sum_j t_j 2^-8j,
@@ -28,7 +27,9 @@
 //
 // lmax 2047 spin 2, one request: 9.7 ms (FP64 recursion throughout, one block
 // of 512 rings per SM: 13.2 ms; two of 256: 12.3 ms; fixed point in half of the
-// warps, to share the work between the FP64 and integer pipes: 9.9 ms).
+// warps, to share the work between the FP64 and integer pipes: 9.9 ms).  At
+// lmax 1023 spin 2 (1.39 ms): issue slots 55 %, ALU pipe 53 %, FP64 pipe 33 %,
+// tensor pipe 7 %; long scoreboard and dependent issue lead the stalls.
 //
 // Layout as in legendre_tc.cu: one order m and 256 rings per block as two
 // 128-row MMA tiles, two blocks per SM, one ring per thread (spin s: 128 pairs,

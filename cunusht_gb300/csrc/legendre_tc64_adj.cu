@@ -25,7 +25,8 @@
 // 0 .. 27).  Two B buffers and four tensor-memory buffers with full / empty
 // mbarriers.  Every wait is bounded; on a timeout the block sets bit 0 of the
 // plan's status word, makes the order's alm NaN (no caller polls that word) and
-// returns.
+// returns.  The ring warps bound it (lmax 1023 spin 2, 2.21 ms: issue slots 41
+// %, ALU pipe 47 %, FP64 pipe 26 %, tensor pipe 15 %, one block of 11 warps per SM).
 #include "common.cuh"
 #include "kernels.cuh"
 #include "rec64.cuh"

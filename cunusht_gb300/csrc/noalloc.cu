@@ -8,7 +8,8 @@
 // serves them: the caller passes the alm and the output map, and every
 // intermediate table and buffer lives in one file-scope __device__ array of
 // CUNUSHT_NOALLOC_SCRATCH_BYTES, which every GPU that loads this library holds
-// until the process exits.  It runs the same kernels as cunusht_synthesis.
+// until the process exits.  It runs the kernels of cunusht_synthesis on an FP64 plan with the
+// tensor cores switched off and chirp-z rings.
 #include <algorithm>
 #include <cmath>
 #include <mutex>

@@ -347,8 +347,7 @@ __device__ __forceinline__ bool kahan_f64_int(float x, float c, double &v) {
 // about two fine cells apart (the grid is oversampled by two), so one tap of
 // 32 lanes reads 32 consecutive cells and not every second one.  Adding
 // sum and compensation as one FP64 value halves the atomics.  Four spin-2 maps
-// of 8.4 M points, w = 9: 13.9 -> 10.6 ms (issue slots 41 -> 63 % used, shared
-// memory 74 %).
+// of 8.4 M points, w = 9: 13.9 -> 10.6 ms (issue slots 41 -> 64 % used).
 // FP32 grid (eps > 1e-6): plain FP32 strip sums of both components and one
 // FP32 atomic per strip cell.
 template <typename TG, bool CPLX, int W>

@@ -1,6 +1,6 @@
 // tcgen05 / TMA-bulk / mbarrier helpers (inline PTX) and the integer-digit
 // split shared by the tensor-core Legendre kernels (legendre_tc.cu,
-// legendre_tc_adj.cu).  sm_100a-family only.
+// legendre_tc_adj.cu, legendre_tc64.cu, legendre_tc64_adj.cu).  sm_100a-family only.
 #pragma once
 #include <cstdint>
 

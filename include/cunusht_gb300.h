@@ -134,16 +134,18 @@ int cunusht_plan_ring_transform(const cunusht_plan_t *plan);
  * (grid 1: spins 0 .. max_spin), 84 MB each at lmax 2047.  enable = 0
  * releases one table: its kernels then start every ring at l = max(m, s)
  * (the same result, no chunk skipped); enable = 1 builds it again
- * (allocates).  Synchronises the device.  No reference counterpart.
+ * (allocates).  FP64 plans keep theirs for the plan's life and refuse the call.  Synchronises the device.  No reference counterpart.
  */
 int cunusht_plan_set_start_states(cunusht_plan_t *plan, int grid, int spin, int enable);
 
 /*
- * Mixed precision: the Legendre synthesis (CC synthesis of spin 0 / 1 / 2
- * maps, the deflection synthesis of dlm2pointing, the ring synthesis of the
- * SHT-only mode) runs on the tensor cores (exact integer-digit bf16 products
- * accumulated in tensor memory, enable = 1, the default) or on the CUDA
- * cores in double-float (enable = 0).
+ * The Legendre stages (CC synthesis of spin 0 / 1 / 2 maps, the deflection
+ * synthesis of dlm2pointing, the ring synthesis of the SHT-only mode, the
+ * adjoints) run on the tensor cores (enable = 1, the default: exact
+ * integer-digit products accumulated in tensor memory, four bf16 digits in
+ * mixed plans, seven fp16 digits in FP64 plans) or on the CUDA cores
+ * (enable = 0: double-float in mixed plans, FP64 in FP64 plans).  Spin 0 of FP64
+ * plans below lmax 96 runs on the CUDA cores either way.
  * Both replace the SHTns synthesis of the reference
  * (cunusht/sht/GPU_sht_transformer.py:56-62, :88-97); the switch exists so
  * that the two can be checked against each other.
@@ -172,8 +174,8 @@ int cunusht_plan_set_spreading(cunusht_plan_t *plan, int method, int determinist
 /*
  * Device status word of the plan, read after the plan's work so far has
  * finished (device-wide synchronisation) and then cleared: 0 = fine; bit 0 =
- * a bounded wait inside a tensor-core kernel ran out (the kernel gave up,
- * its outputs are not valid).  No reference counterpart.
+ * a bounded wait inside a tensor-core kernel ran out (the kernel gave up, its
+ * outputs are not valid; FP64 plans return NaN for them).  No reference counterpart.
  */
 int cunusht_plan_device_status(cunusht_plan_t *plan, int *status);
 
