@@ -20,9 +20,9 @@
 namespace cunusht {
 
 // One weight, out of line: 2 W copies in each of the 30 kernels below would triple the compile time
-// (a call costs about a tenth of the 110 instructions it makes).
-static __device__ __noinline__ double es_weight64(dfl f0, float a, dfl s, dfl nbeta, const float2 *T) {
-    return df_to(es_kernel_df<false>(f0, a, EsParams{s, nbeta}, T, nullptr));
+// (a call costs about a tenth of the 120 instructions it makes).
+static __device__ __noinline__ double es_weight64(dfl f0, float a, dfl s, dfl nbeta, float hw, const float2 *T) {
+    return df_to(es_kernel_df<false>(f0, a, EsParams{s, nbeta, hw}, T, nullptr));
 }
 
 // FP64 kernel weights of the W taps per axis: the split evaluation up to
@@ -30,12 +30,12 @@ static __device__ __noinline__ double es_weight64(dfl f0, float a, dfl s, dfl nb
 template <int W>
 __device__ __forceinline__ void weights64(const PointCoords &pc, double beta, const float2 *T, double *kt, double *kp) {
     if constexpr (W <= ES_SPLIT_MAXW) {
-        const EsParams E{df_from(2.0 / W), df_from(-beta)};
+        const EsParams E{df_from(2.0 / W), df_from(-beta), 0.5f * W};
         const dfl ft = df_from(pc.ft), fp = df_from(pc.fp);
 #pragma unroll
         for (int a = 0; a < W; ++a) {
-            kt[a] = es_weight64(ft, (float)a, E.s, E.nbeta, T);
-            kp[a] = es_weight64(fp, (float)a, E.s, E.nbeta, T);
+            kt[a] = es_weight64(ft, (float)a, E.s, E.nbeta, E.hw, T);
+            kp[a] = es_weight64(fp, (float)a, E.s, E.nbeta, E.hw, T);
         }
     } else {
         const double s = 2.0 / W;
@@ -1031,7 +1031,7 @@ __global__ void __launch_bounds__(256)
     const double sc = 2.0 / w;
     const double dzt = -sc * Ntf / TWOPI, dzp = -sc * Npf / TWOPI;  // dz / dtheta, dz / dphi
     if (w <= ES_SPLIT_MAXW) {
-        const EsParams E{df_from(sc), df_from(-beta)};
+        const EsParams E{df_from(sc), df_from(-beta), 0.5f * w};
         const dfl f0 = df_from(pc.ft), f1 = df_from(pc.fp);
 #pragma unroll 1
         for (int a = 0; a < w; ++a) {

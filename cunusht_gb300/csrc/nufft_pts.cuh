@@ -165,12 +165,12 @@ __device__ const float2 ES_EXP2[128] = {
     {0x1.fa7c18p+0f, 0x1.9e90d8p-28f}, {0x1.fd3c22p+0f, 0x1.71ee3ep-25f}};
 
 // The kernel value of the FP64 plans from double-float arithmetic on the FP32
-// pipe: about 100 FP32 instructions for the value (absolute error up to 2.4e-14, of
+// pipe: about 115 FP32 instructions for the value (absolute error up to 2.4e-14, of
 // values up to 1) in place of about 33 FP64 instructions of exp, sqrt and
 // products, each of which takes the issue time of 64 (2 FP64 lanes per SM and
 // clock, measured).  z = (a + f) s with f the offset of the first tap and s =
-// 2 / w; exponent y = -beta z^2 / (1 + sqrt(1 - z^2)) (no cancellation); e^y =
-// 2^k (2^(j/128)) e^f from the table T in shared memory with |f| < 0.0028, ln 2
+// 2 / w; u = 1 - |z|, q = 1 - z^2 = u (2 - u); exponent y = -beta z^2 / (1 + sqrt(q)) (no
+// cancellation); e^y = 2^k (2^(j/128)) e^f from the table T in shared memory with |f| < 0.0028, ln 2
 // / 128 split so that the first two products are exact.  Used for widths up to
 // ES_SPLIT_MAXW (eps >= 1e-10), where the kernel's own aliasing error is over a
 // hundred times larger (with FP64 weights the errors of both transform types and of
@@ -179,13 +179,17 @@ __device__ const float2 ES_EXP2[128] = {
 constexpr int ES_SPLIT_MAXW = 12;
 struct EsParams {
     dfl s, nbeta;  // 2 / w, -beta
+    float hw;      // w / 2
 };
 template <bool DERIV>
 __device__ __forceinline__ dfl es_kernel_df(dfl f0, float a, const EsParams &E, const float2 *T, dfl *dlog) {
-    const dfl z = df_mul(df_add(dfl{a, 0.f}, f0), E.s);
+    const dfl x = df_add(dfl{a, 0.f}, f0);
+    const dfl z = df_mul(x, E.s);
     const dfl z2 = df_mul(z, z);
-    dfl q = df_fast(1.f, -z2.h);
-    q = df_fast(q.h, q.l - z2.l);
+    // u = 1 - |z| from the distance to the kernel's edge, exact: zero there (1 - z^2 of the
+    // rounded z is up to 2e-15, where the derivative's 1 / sqrt(q) is at its largest)
+    const dfl u = df_mul(df_add(dfl{E.hw, 0.f}, x.h < 0.f ? x : df_neg(x)), E.s);
+    const dfl q = df_mul(u, df_add(dfl{2.f, 0.f}, df_neg(u)));
     if (DERIV) *dlog = dfl{0.f, 0.f};
     if (!(q.h > 0.f)) return dfl{0.f, 0.f};
     const float r0 = sqrtf(q.h);
