@@ -22,7 +22,7 @@ namespace cunusht {
 // One weight, out of line: 2 W copies in each of the 30 kernels below would triple the compile time
 // (a call costs about a tenth of the 120 instructions it makes).
 static __device__ __noinline__ double es_weight64(dfl f0, float a, dfl s, dfl nbeta, float hw, const float2 *T) {
-    return df_to(es_kernel_df<false>(f0, a, EsParams{s, nbeta, hw}, T, nullptr));
+    return df_to(es_kernel_df<false>(f0, a, EsParams{s, nbeta, hw, 0.f}, T, nullptr));
 }
 
 // FP64 kernel weights of the W taps per axis: the split evaluation up to
@@ -30,7 +30,7 @@ static __device__ __noinline__ double es_weight64(dfl f0, float a, dfl s, dfl nb
 template <int W>
 __device__ __forceinline__ void weights64(const PointCoords &pc, double beta, const float2 *T, double *kt, double *kp) {
     if constexpr (W <= ES_SPLIT_MAXW) {
-        const EsParams E{df_from(2.0 / W), df_from(-beta), 0.5f * W};
+        const EsParams E{df_from(2.0 / W), df_from(-beta), 0.5f * W, 0.f};
         const dfl ft = df_from(pc.ft), fp = df_from(pc.fp);
 #pragma unroll
         for (int a = 0; a < W; ++a) {
@@ -1030,15 +1030,21 @@ __global__ void __launch_bounds__(256)
     double kt[MAXW], dkt[MAXW], kp[MAXW], dkp[MAXW];
     const double sc = 2.0 / w;
     const double dzt = -sc * Ntf / TWOPI, dzp = -sc * Npf / TWOPI;  // dz / dtheta, dz / dphi
+    // A tap whose distance to the kernel's edge is within the coordinates' rounding (8 units) counts as
+    // on the edge, where the derivative is left out: it grows as 1 / sqrt(1 - z^2), and points that stay
+    // on a column of the fine grid (zero deflection on HEALPix or power-of-two rings) would have
+    // gradients of any size there (27 % off at w = 8)
+    const double edge_t = 0x1p-50 * Ntf * sc, edge_p = 0x1p-50 * Npf * sc;
     if (w <= ES_SPLIT_MAXW) {
-        const EsParams E{df_from(sc), df_from(-beta), 0.5f * w};
+        EsParams E{df_from(sc), df_from(-beta), 0.5f * w, (float)edge_t}, Ep = E;
+        Ep.edge = (float)edge_p;
         const dfl f0 = df_from(pc.ft), f1 = df_from(pc.fp);
 #pragma unroll 1
         for (int a = 0; a < w; ++a) {
             dfl g, v = es_kernel_df<true>(f0, (float)a, E, s_exp2, &g);
             kt[a] = df_to(v);
             dkt[a] = df_to(df_mul(v, g)) * dzt;
-            v = es_kernel_df<true>(f1, (float)a, E, s_exp2, &g);
+            v = es_kernel_df<true>(f1, (float)a, Ep, s_exp2, &g);
             kp[a] = df_to(v);
             dkp[a] = df_to(df_mul(v, g)) * dzp;
         }
@@ -1050,8 +1056,8 @@ __global__ void __launch_bounds__(256)
             const double rt = qt > 0.0 ? sqrt(qt) : 0.0, rp = qp > 0.0 ? sqrt(qp) : 0.0;
             kt[a] = qt > 0.0 ? exp(beta * (rt - 1.0)) : 0.0;
             kp[a] = qp > 0.0 ? exp(beta * (rp - 1.0)) : 0.0;
-            dkt[a] = qt > 1e-24 ? kt[a] * (-beta * zt / rt) * dzt : 0.0;
-            dkp[a] = qp > 1e-24 ? kp[a] * (-beta * zp / rp) * dzp : 0.0;
+            dkt[a] = qt > 2.0 * edge_t ? kt[a] * (-beta * zt / rt) * dzt : 0.0;
+            dkp[a] = qp > 2.0 * edge_p ? kp[a] * (-beta * zp / rp) * dzp : 0.0;
         }
     }
     double ft = 0.0, fp = 0.0;

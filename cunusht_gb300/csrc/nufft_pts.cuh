@@ -180,6 +180,7 @@ constexpr int ES_SPLIT_MAXW = 12;
 struct EsParams {
     dfl s, nbeta;  // 2 / w, -beta
     float hw;      // w / 2
+    float edge;    // derivatives: 1 - |z| up to here counts as 0
 };
 template <bool DERIV>
 __device__ __forceinline__ dfl es_kernel_df(dfl f0, float a, const EsParams &E, const float2 *T, dfl *dlog) {
@@ -200,7 +201,7 @@ __device__ __forceinline__ dfl es_kernel_df(dfl f0, float a, const EsParams &E, 
     const float i0 = 1.f / d.h;
     const float y0 = bz.h * i0;
     const dfl y = df_fast(y0, (fmaf(-y0, d.l, fmaf(-y0, d.h, bz.h)) + bz.l) * i0);
-    if (DERIV) {  // d log(psi) / dz = -beta z / sqrt(1 - z^2)
+    if (DERIV && u.h > E.edge) {  // d log(psi) / dz = -beta z / sqrt(1 - z^2)
         const dfl n = df_mul(E.nbeta, z);
         const float g0 = n.h / r.h;
         *dlog = df_fast(g0, (fmaf(-g0, r.l, fmaf(-g0, r.h, n.h)) + n.l) / r.h);

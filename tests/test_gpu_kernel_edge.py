@@ -56,3 +56,17 @@ def test_spreading_from_grid_columns(built_lib, eps, spin):
     t.set_spreading("bins", max_points=n)
     y = t.nusht2d1(lmax, lmax, v, loc, spin=spin)
     assert float((x - y).norm() / y.norm()) < 1e-12
+
+
+# rings whose pixels all lie on grid columns, up to rounding
+@pytest.mark.parametrize("geom", [("gl", {"lmax": 63, "nphi": 128}), ("healpix", {"nside": 32, "lmax": 64}),
+                                  ("f1", {"ntheta": 70, "nphi": 128, "lmax": 63})])
+@pytest.mark.parametrize("eps", [1e-4, 1e-6, 1e-8, 1e-10, 1e-12])
+def test_deflection_gradient_on_aligned_rings(built_lib, geom, eps):
+    """Zero deflection: every pixel stays on a column, its edge tap within the
+    rounding of phi of |z| = 1 (widths 6 to 14; the last has FP64 weights)."""
+    import cunusht_gb300 as cu
+    lmax = geom[1]["lmax"]
+    x, ref = [_grad(cu.get_transformer("GPU")(geom, nuFFTtype=2, epsilon=e, precision="fp64", max_spin=2), lmax)
+              for e in (eps, 1e-13)]
+    assert float((x - ref).norm() / ref.norm()) < 100 * eps
