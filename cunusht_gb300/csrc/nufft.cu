@@ -789,7 +789,7 @@ int nufft_spread(const cunusht_plan_s *P, int spin, const double *loc, long long
 // difference (equal modulo 2 pi).
 // geo (may be NULL): per ring sin, cos, cot of the colatitude and the pixel spacing, from the plan.
 // FP64 instructions bound it: about 330 per pixel with sincos, three atan2 and the divisions by
-// constants, about 100 with ring tables and series of the increments; 8.4 M pixels 4.46 -> 1.35 ms.
+// constants, about 100 with ring tables and series of the increments; 8.4 M pixels 4.46 -> 1.32 ms.
 __device__ __forceinline__ double asin_small(double x) {  // |x| < 0.02: error below 1e-20
     const double x2 = x * x;
     return x + x * x2 * (1.0 / 6.0 + x2 * (3.0 / 40.0 + x2 * (15.0 / 336.0 + x2 * (105.0 / 3456.0))));
@@ -857,9 +857,12 @@ __global__ void __launch_bounds__(256)
     const double rho = sqrt(nx * nx + ny * ny);
     // the increments from their series where they are small (all but the pixels next to a pole):
     // theta' - theta = asin(rho ct - nz st), phi' - phi = -atan(ny / nx).  The sine is as small where
-    // a pixel next to one pole moves next to the other: there the cosine is negative
-    const double sd = rho * ct - nz * st, cd = rho * st + nz * ct;
-    oth[j] = fabs(sd) < 0.02 && cd > 0.0 ? theta + asin_small(sd) : atan2(rho, nz);
+    // a pixel next to one pole moves next to the other: there nz and ct differ in sign and are not
+    // small (a test of their high words; the cosine itself, two FP64 instructions: 1.36 ms for 1.32)
+    const double sd = rho * ct - nz * st;
+    const int hz = __double2hiint(nz), hc = __double2hiint(ct);
+    const bool near = (hz ^ hc) >= 0 || (hc & 0x7fffffff) < 0x3fe00000;  // same sign, or |ct| < 1/2
+    oth[j] = fabs(sd) < 0.02 && near ? theta + asin_small(sd) : atan2(rho, nz);
     const double q = ny / nx;
     double php = phi - (nx > 0.0 && fabs(q) < 0.02 ? atan_small(q) : atan2(ny, nx));
     if (php >= TWOPI) php -= TWOPI;
